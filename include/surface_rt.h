@@ -129,7 +129,7 @@ typedef struct srt_trace_opts {
    * as BuildIntersection computes it) */
   float *normal_out;
   /* work counters (device memory, 4 x uint64, accumulated): branch nodes
-   * visited, leaves visited, primitive tests -- the reference's
+   * visited (a wide node counts once), leaves visited, primitive tests -- the reference's
    * TetraTraversalStatistics (render/render_accel_tetra.h:70-78) -- and
    * rays that took the reference's walk */
   unsigned long long *stats;

@@ -298,7 +298,7 @@ __device__ __forceinline__ SceneInfo scene_of_box(const Box &r) {
     s.keps = FLT_EPSILON * 16;
   }
   s.nbranches = 0;
-  s.pad = 0;
+  s.irregular = 0;
   return s;
 }
 
@@ -1190,6 +1190,21 @@ __global__ void emit_node2_kernel(const uint32_t *__restrict__ codes,
   }
 }
 
+// One child of a two-child node; count 0: a branch.
+struct Box2 {
+  float lo[3], hi[3];
+  uint32_t ref, count;
+};
+__device__ __forceinline__ Box2 node2_child(const Node2 &n, uint32_t side) {
+  Box2 c;
+  if (side == 0) {
+    c = Box2{{n.a.x, n.a.y, n.a.z}, {n.a.w, n.b.x, n.b.y}, n.d.x, n.d.z & kCountMask};
+  } else {
+    c = Box2{{n.b.z, n.b.w, n.c.x}, {n.c.y, n.c.z, n.c.w}, n.d.y, n.d.w & kCountMask};
+  }
+  return c;
+}
+
 __device__ __forceinline__ NodeT make_tet_node(const Box &b, uint32_t meta, uint32_t ref) {
   NodeT t;
   t.a = make_float4(b.lo[0], b.lo[1], b.lo[2], __uint_as_float(meta));
@@ -1243,6 +1258,36 @@ __global__ void emit_tet_kernel(const uint32_t *__restrict__ codes,
 }
 
 
+// The wide nodes (WideRec) of the two-child nodes, a thread per record.
+// Memory bound and small: 128 bytes written and up to 192 read per branch
+// (most of it shared by the branch's four threads), 1/12 as many branches
+// as primitives.
+__global__ void widen_kernel(const Node2 *__restrict__ nodes,
+                             const uint32_t *__restrict__ nbranches, uint32_t cap,
+                             WideRec *__restrict__ wide, uint32_t *__restrict__ irregular) {
+  const uint32_t nb = *nbranches;
+  if (nb > cap) return;  // the two-child nodes are walked instead
+  for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < 4 * nb;
+       t += gridDim.x * blockDim.x) {
+    const Box2 p = node2_child(nodes[t >> 2], (t >> 1) & 1u);
+    Box2 q = p;
+    if (p.count == 0) {
+      q = node2_child(nodes[p.ref], t & 1u);
+    } else if (t & 1u) {
+      q.count = kNone;
+    }
+    bool ok = true;
+#pragma unroll
+    for (int k = 0; k < 3; k++)
+      ok = ok && p.lo[k] <= q.lo[k] && q.lo[k] <= q.hi[k] && q.hi[k] <= p.hi[k];
+    if (!ok) *irregular = 1u;
+    WideRec r;
+    r.a = make_float4(q.lo[0], q.hi[0], q.lo[1], q.hi[1]);
+    r.b = make_float4(q.lo[2], q.hi[2], __uint_as_float(q.ref), __uint_as_float(q.count));
+    wide[t] = r;
+  }
+}
+
 // Scene box and Morton codes.  With `hist` (3 x 1024 words) and `tickets`,
 // also the digit histograms of sort_codes30's passes (hist_ready).
 template <int KIND>
@@ -1275,6 +1320,25 @@ srt_status launch_bbox_morton(srt_ctx *ctx, const float *v, const uint32_t *f,
 
 constexpr size_t kOneSweepMax = (size_t)1 << 18;
 
+// Wide nodes allocated for a tree over n primitives: up to kWideAll (32 MB)
+// one for every branch that any tree could have, above that a sixth of them
+// -- a branch has 18 primitives or more below it, an emitted tree about one
+// branch per 12 primitives -- and a tree with more is walked by its
+// two-child nodes.
+constexpr size_t kWideAll = (size_t)1 << 18;
+uint32_t wide_slots(size_t n) {
+  return (uint32_t)std::max<size_t>(std::min(n - 1, kWideAll), (n - 1) / 6);
+}
+// Wide nodes of an emitted tree (nbranches: a device word) over m internal
+// Karras nodes.
+srt_status build_wide(srt_ctx *ctx, const Node2 *nodes, const uint32_t *nbranches, size_t m,
+                      uint32_t cap, WideRec *wide, uint32_t *irregular) {
+  const int g = grid_for(std::min<size_t>(m, cap) / 2 + 1, kBlock, ctx->num_sms * 8);
+  widen_kernel<<<g, kBlock, 0, ctx->stream>>>(nodes, nbranches, cap, wide, irregular);
+  ctx->launches++;
+  return cuda_status(cudaGetLastError(), "wide nodes");
+}
+
 template <int KIND>
 srt_status build_kind(srt_accel *a, const float *v, const uint32_t *f,
                       const float *radius, float constr, size_t n) {
@@ -1294,6 +1358,11 @@ srt_status build_kind(srt_accel *a, const float *v, const uint32_t *f,
   ENSURE(a->scene, sizeof(SceneInfo));
   size_t max_nodes = (KIND == SRT_TETRAHEDRA) ? (2 * m + 1) : m;
   ENSURE(a->nodes, max_nodes * (KIND == SRT_TETRAHEDRA ? sizeof(NodeT) : sizeof(Node2)));
+  if (KIND != SRT_TETRAHEDRA) {
+    a->wide_cap = wide_slots(n);
+    a->wide_all = a->wide_cap >= m;
+    ENSURE(a->wide, (size_t)a->wide_cap * 4 * sizeof(WideRec));
+  }
 
   ENSURE(ctx->s_kchild, m * 4);
   ENSURE(ctx->s_kflags, m);
@@ -1382,6 +1451,9 @@ srt_status build_kind(srt_accel *a, const float *v, const uint32_t *f,
                                                    scene, kidx, a->nodes.as<Node2>(),
                                                    ctx->d_err);
     ctx->launches++;
+    s = build_wide(ctx, a->nodes.as<Node2>(), &scene->nbranches, m, a->wide_cap,
+                   a->wide.as<WideRec>(), &scene->irregular);
+    if (s != SRT_OK) return s;
   }
 #undef ENSURE2
   return cuda_status(cudaGetLastError(), "emit");
@@ -1543,7 +1615,7 @@ __global__ void seg_finalize_kernel(const int *__restrict__ acc, int nseg,
     si.keps = FLT_EPSILON * 16;
   }
   si.nbranches = 0;
-  si.pad = 0;
+  si.irregular = 0;
   scenes[sg] = si;
 }
 
@@ -1872,6 +1944,7 @@ __global__ void gather_codes_kernel(const uint32_t *__restrict__ codes,
 
 __global__ void set_branches_kernel(SceneInfo *__restrict__ scene, uint32_t nb) {
   scene->nbranches = nb;
+  scene->irregular = 0;
 }
 
 // An accel from a tree read from a file: the scene box and codes as the build
@@ -1906,6 +1979,15 @@ srt_status load_kind(srt_accel *a, const float *v, const uint32_t *f, const floa
                                            a->prims.as<float4>());
   set_branches_kernel<<<1, 1, 0, st>>>(scene, nbranches);
   ctx->launches += 3;
+  if (KIND != SRT_TETRAHEDRA) {
+    a->wide_cap = nbranches;
+    a->wide_all = true;
+    if ((e = a->wide.ensure((size_t)nbranches * 4 * sizeof(WideRec))) != cudaSuccess)
+      return cuda_status(e, "load allocation");
+    s = build_wide(ctx, a->nodes.as<Node2>(), &scene->nbranches, nbranches, nbranches,
+                   a->wide.as<WideRec>(), &scene->irregular);
+    if (s != SRT_OK) return s;
+  }
   if ((e = cudaGetLastError()) != cudaSuccess) return cuda_status(e, "load");
   // the host arrays are the caller's until the copies are done
   return cuda_status(cudaStreamSynchronize(st), "load");

@@ -48,6 +48,19 @@ struct __align__(16) Node2 {
   uint4 d;
 };
 
+// Wide node: the four grandchildren of a branch, one 32-byte record each, so
+// that four lanes that share a ray read one 128-byte line and test one box
+// each.  Record k of branch b (slot 4 b + k): grandchild k & 1 of child
+// k >> 1; a leaf child takes record 2 (k >> 1) and leaves the next one empty.
+//   a = (lo.x, hi.x, lo.y, hi.y), b = (lo.z, hi.z, ref, count)
+// count = a leaf's primitive count (ref its first sorted primitive), 0 for a
+// branch (ref its node index), kNone for an empty record.
+struct __align__(32) WideRec {
+  float4 a, b;
+};
+// SceneInfo.irregular: some box of the wide nodes is not ordered (lo <= hi,
+// false for NaN) or not inside its parent's.
+
 // Own-box node (tetrahedra): 32 bytes, the reference's TetraNode.
 //   a = (lo.x, lo.y, lo.z, meta)  meta: leaf -> kLeafBit | count, branch -> axis
 //   b = (hi.x, hi.y, hi.z, ref)   ref:  leaf -> first sorted primitive,
@@ -63,7 +76,7 @@ struct SceneInfo {
   float keps;        // leaf box padding
   double eps_scale;  // triangles: max scene extent
   uint32_t nbranches;
-  uint32_t pad;
+  uint32_t irregular;  // see WideRec
 };
 
 struct Box {
@@ -195,6 +208,12 @@ struct srt_accel {
   size_t nnodes_cap = 0;
   bool built = false;
   srt::DevBuf nodes, indices, codes, prims, scene;
+  // wide nodes of the tree's first wide_cap branches (a tree with more
+  // branches is walked by its two-child nodes alone); wide_all: it has none
+  // beyond them whatever its shape
+  srt::DevBuf wide;
+  uint32_t wide_cap = 0;
+  bool wide_all = false;
   srt::DevBuf in_verts, in_faces, in_radius;  // device copies of host inputs
   // primitive arrays the tree was built from (owned copies of host inputs,
   // or the caller's device arrays, borrowed like the reference's mesh_)

@@ -42,16 +42,11 @@ struct RayF {
   int sgn[3];
 };
 
-__device__ __forceinline__ RayF load_ray(const srt_ray *__restrict__ rays, size_t i,
-                                         uint32_t &prev_prim, float &prev_t) {
-  const float4 *r4 = reinterpret_cast<const float4 *>(rays + i);
-  float4 a = __ldg(&r4[0]);
-  float4 b = __ldg(&r4[1]);
+// A ray of its record's two words.
+__device__ __forceinline__ RayF ray_of(float4 a, float4 b) {
   RayF r;
   r.o[0] = a.x; r.o[1] = a.y; r.o[2] = a.z;
   r.d[0] = b.x; r.d[1] = b.y; r.d[2] = b.z;
-  prev_prim = __float_as_uint(a.w);
-  prev_t = b.w;
 #pragma unroll
   for (int k = 0; k < 3; k++) {
     r.sgn[k] = r.d[k] < 0.0f ? 1 : 0;
@@ -59,6 +54,16 @@ __device__ __forceinline__ RayF load_ray(const srt_ray *__restrict__ rays, size_
     r.inv[k] = __frcp_rn(r.d[k]);
   }
   return r;
+}
+
+__device__ __forceinline__ RayF load_ray(const srt_ray *__restrict__ rays, size_t i,
+                                         uint32_t &prev_prim, float &prev_t) {
+  const float4 *r4 = reinterpret_cast<const float4 *>(rays + i);
+  const float4 a = __ldg(&r4[0]);
+  const float4 b = __ldg(&r4[1]);
+  prev_prim = __float_as_uint(a.w);
+  prev_t = b.w;
+  return ray_of(a, b);
 }
 
 // IntersectRayAABB; CLAMP: tmax = min(tmax, maxT) (triangle/particle) else
@@ -322,6 +327,17 @@ __device__ __forceinline__ bool sphere_isect(float &tio, const float c[3], float
     return true;
   }
   return false;
+}
+
+// False only if sphere_isect's discriminant is negative: b and cc are its
+// own floats and b^2 - 4 a cc formed from them in float is off by less than
+// 2^-22 (b^2 + |4 a cc|) (four roundings of 2^-24 each); NaN counts as maybe.
+__device__ __forceinline__ bool sphere_maybe(const float4 s, const RayF &r, float a) {
+  const float oc[3] = {r.o[0] - s.x, r.o[1] - s.y, r.o[2] - s.z};
+  const float b = 2.0f * dot3(r.d, oc);
+  const float cc = dot3(oc, oc) - s.w * s.w;
+  const float bb = b * b, q = 4.0f * a * cc;
+  return !(bb - q < -2.3841858e-7f * (bb + fabsf(q)));
 }
 
 // real3::normalize (render/render_common.h:64-77): length in double.
@@ -816,6 +832,378 @@ __device__ __forceinline__ void pass1_node2(const Node2 *__restrict__ nodes,
   viol_out = viol;
 }
 
+// --------------------------------------------------------------- wide walk
+// Pass 1 with four lanes per ray (a group) over the wide nodes.  One thread
+// per ray is bound by its dependent chain -- about 18 nodes and 19 primitives
+// one after the other -- and by divergence (12.7 of 32 lanes active per
+// instruction); four lanes test four grandchildren or four primitives of a
+// leaf at once, so the chain is less than half as long, a warp holds 8 rays
+// instead of 32 to diverge, and every node read is one 128-byte line.
+// A leaf is entered exactly when pass1_node2 enters it for the same bound:
+// the boxes of regular trees nest and the slab arithmetic is monotone, so a
+// ray that enters a grandchild's box enters the child's no later.  Where that
+// does not hold (a zero, infinite or NaN ray component, whose products can be
+// NaN; boxes that do not nest) the child's box is tested too, with the
+// reference's comparisons.
+constexpr int kGrp = 4;
+// Entries of a group's stack, (node or leaf record, box entry distance): a
+// visit pops one and pushes at most four, 12 levels of wide nodes in a built
+// tree (branches lie at levels 0 to 23) and 14 in a loaded one.  A group's
+// entries lie together; an odd number of them puts the eight groups of a
+// warp on different banks at equal depths.
+constexpr int kWideStack = 45;
+
+template <int KIND>
+struct WideTree {
+  const WideRec *wide;
+  const Node2 *nodes;
+  const float4 *prims;
+  const uint32_t *sidx;
+  bool irregular;
+};
+
+// The lanes of this thread's group.  The groups of a warp advance together,
+// idle ones predicated off: every exchange is a full-warp shuffle or vote
+// (exchanges among diverged groups cost a reconvergence each).
+struct Group {
+  int lane, shift;  // 0..3, first lane in the warp
+  __device__ __forceinline__ Group() {
+    lane = (int)(threadIdx.x & 3u);
+    shift = (int)(threadIdx.x & 28u);
+  }
+  template <typename T>
+  __device__ __forceinline__ T other(T v, int x) const {
+    return __shfl_xor_sync(0xffffffffu, v, x);
+  }
+  // this group's bits of a full-warp vote
+  __device__ __forceinline__ unsigned vote(bool p) const {
+    return (__ballot_sync(0xffffffffu, p) >> shift) & 0xfu;
+  }
+  __device__ __forceinline__ float min4(float v) const {
+    v = fminf(v, other(v, 1));
+    return fminf(v, other(v, 2));
+  }
+};
+
+// Two floats as one 64-bit operand of the packed instructions: each half is
+// added and multiplied with its own IEEE rounding.
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  unsigned long long r;
+  asm("add.rn.f32x2 %0, %1, %2;"
+      : "=l"(r)
+      : "l"(*reinterpret_cast<unsigned long long *>(&a)),
+        "l"(*reinterpret_cast<unsigned long long *>(&b)));
+  return *reinterpret_cast<float2 *>(&r);
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  unsigned long long r;
+  asm("mul.rn.f32x2 %0, %1, %2;"
+      : "=l"(r)
+      : "l"(*reinterpret_cast<unsigned long long *>(&a)),
+        "l"(*reinterpret_cast<unsigned long long *>(&b)));
+  return *reinterpret_cast<float2 *>(&r);
+}
+
+// A component the slab test's products can turn into NaN.
+__device__ __forceinline__ bool odd_ray(const RayF &r) {
+  bool odd = false;
+#pragma unroll
+  for (int k = 0; k < 3; k++)
+    odd = odd || !(fabsf(r.o[k]) <= FLT_MAX) || !(fabsf(r.inv[k]) <= FLT_MAX) || r.inv[k] == 0.0f;
+  return odd;
+}
+
+// A lane's candidates: the smallest distance m with its barycentrics and
+// sorted primitive, its leaf box's entry, the second smallest distance, and
+// whether another primitive lies at m (and one of those below its box).
+struct Cand {
+  float m = FLT_MAX, m2 = FLT_MAX, u = 0.0f, v = 0.0f, e = 0.0f;
+  uint32_t j = kNone;
+  bool tie = false, tie_viol = false;
+  __device__ __forceinline__ void take(float t, float uu, float vv, uint32_t jj, float entry) {
+    if (t < m) {
+      m2 = m;
+      m = t;
+      u = uu;
+      v = vv;
+      j = jj;
+      e = entry;
+      tie = tie_viol = false;
+    } else {
+      m2 = fminf(m2, t);
+      if (t == m) {
+        tie = true;
+        tie_viol = tie_viol || below_entry(t, entry);
+      }
+    }
+  }
+};
+
+// The outcome of a group's pass: what pass1_node2 reports, and the lane
+// (of the warp) that holds the primitive found.
+struct WidePass {
+  bool defer, viol;
+  int winner;
+};
+
+// stk: the group's stack.  Called by the whole warp; live: the group has a ray.
+template <int KIND, int DEPTH = kWideStack>
+__device__ __forceinline__ WidePass pass1_wide(const WideTree<KIND> &T, const Group &G,
+                                               const Ctx2 &c, uint32_t root, bool live,
+                                               uint2 *stk, Cand &C, Work &w,
+                                               uint32_t max_iter) {
+  constexpr unsigned kAll = 0xffffffffu;
+  const bool odd = T.irregular || odd_ray(c.r);
+  const float2 nox = make_float2(-c.r.o[0], -c.r.o[0]), noy = make_float2(-c.r.o[1], -c.r.o[1]),
+               noz = make_float2(-c.r.o[2], -c.r.o[2]);
+  const float2 ivx = make_float2(c.r.inv[0], c.r.inv[0]), ivy = make_float2(c.r.inv[1], c.r.inv[1]),
+               ivz = make_float2(c.r.inv[2], c.r.inv[2]);
+  const float ray_a = dot3(c.r.d, c.r.d);
+  float bnd = FLT_MAX;  // the group's pruning bound
+  int sp = live ? 1 : 0;
+  if (live && G.lane == 0) stk[0] = make_uint2(root, __float_as_uint(-FLT_MAX));
+  __syncwarp();
+  while (true) {
+    // down to the next leaf of every group that has one
+    uint32_t leaf = kNone;
+    float lt = 0.0f;
+    while (__any_sync(kAll, sp > 0 && leaf == kNone)) {
+      const bool go = sp > 0 && leaf == kNone;
+      uint2 e = make_uint2(0u, 0x7f800000u);
+      if (go) e = stk[sp - 1];
+      sp -= go ? 1 : 0;
+      const float et = __uint_as_float(e.y);
+      const bool in = et <= bnd;
+      const bool lf = in && (int)e.x < 0;
+      if (lf) leaf = e.x & ~kLeafBit;
+      if (lf) lt = et;
+      const bool visit = in && !lf;
+      const uint32_t slot = 4 * e.x + (uint32_t)G.lane;
+      float4 A, B = make_float4(0.f, 0.f, 0.f, __uint_as_float(kNone));
+      if (visit) {
+        const float4 *rp = reinterpret_cast<const float4 *>(T.wide + slot);
+        A = __ldg(rp);
+        B = __ldg(rp + 1);
+      }
+      w.it += visit ? 1u : 0u;
+      const uint32_t count = __float_as_uint(B.w);
+      const float2 x = mul2(add2(make_float2(A.x, A.y), nox), ivx);
+      const float2 y = mul2(add2(make_float2(A.z, A.w), noy), ivy);
+      const float2 z = mul2(add2(make_float2(B.x, B.y), noz), ivz);
+      float tmin = fmaxf(fmaxf(fminf(x.x, x.y), fminf(y.x, y.y)), fminf(z.x, z.y));
+      const float tmax = fminf(fminf(fmaxf(x.x, x.y), fmaxf(y.x, y.y)), fmaxf(z.x, z.y));
+      bool hit = tmax > 0.0f && tmin <= fminf(tmax, bnd) && count != kNone;
+      if (odd && visit && count != kNone) {
+        hit = ray_aabb_t<true>(bnd, A.x, A.z, B.x, A.y, A.w, B.y, c.r, tmin);
+        const float4 *np = reinterpret_cast<const float4 *>(T.nodes + e.x);
+        const float4 a = __ldg(np), bb = __ldg(np + 1), cc = __ldg(np + 2);
+        if (G.lane < 2)
+          hit = hit && ray_aabb<true>(bnd, a.x, a.y, a.z, a.w, bb.x, bb.y, c.r);
+        else
+          hit = hit && ray_aabb<true>(bnd, bb.z, bb.w, cc.x, cc.y, cc.z, cc.w, c.r);
+      }
+      // nearest entry on top: the rank among the group's hits by distance
+      // (to a quarter of its low bits: order only), then lane
+      const int key = hit ? (__float_as_int(fmaxf(tmin, 0.0f)) & ~3) | G.lane : INT_MAX;
+      const int k1 = G.other(key, 1), k2 = G.other(key, 2), k3 = G.other(key, 3);
+      const int nh = __popc(G.vote(hit));
+      const int rank = (k1 < key) + (k2 < key) + (k3 < key);
+      const int top = sp + nh;
+      if (top > DEPTH || w.it > max_iter) {
+        w.fail = true;
+        sp = 0;
+        hit = false;
+      } else {
+        sp = top;
+      }
+      if (hit)
+        stk[top - 1 - rank] = make_uint2(count ? kLeafBit | slot : __float_as_uint(B.z),
+                                                __float_as_uint(tmin));
+      __syncwarp();
+    }
+    if (!__any_sync(kAll, leaf != kNone)) break;
+    uint32_t j = 0, end = 0;
+    if (leaf != kNone) {
+      const uint2 rc = __ldg(reinterpret_cast<const uint2 *>(T.wide + leaf) + 3);
+      j = rc.x + (uint32_t)G.lane;
+      end = rc.x + rc.y;
+      w.leaf++;
+      w.prim += rc.y;
+    }
+    if (KIND == SRT_TRIANGLES) {
+      for (; j < end; j += kGrp) {
+        Prim2<KIND> P;
+        P.load(T.prims, T.sidx, j);
+        float t, u, v;
+        if (P.test(c, FLT_MAX, t, u, v)) C.take(t, u, v, j, lt);
+      }
+    } else {
+      // most spheres of a leaf are missed: those whose discriminant is surely
+      // negative are dropped first, so that the square root and divisions run
+      // once or twice per leaf instead of for every sphere
+      while (__any_sync(kAll, j < end)) {
+        unsigned maybe = 0;
+        const uint32_t j0 = j;
+        for (int q = 0; q < 8 && j < end; q++, j += kGrp)
+          if (sphere_maybe(__ldg(&T.prims[j]), c.r, ray_a)) maybe |= 1u << q;
+        while (maybe) {
+          const uint32_t jj = j0 + kGrp * (uint32_t)(__ffs(maybe) - 1);
+          maybe &= maybe - 1;
+          const float4 q = __ldg(&T.prims[jj]);
+          const bool self = c.prev_prim != kNone && __ldg(&T.sidx[jj]) == c.prev_prim;
+          const float c3[3] = {q.x, q.y, q.z};
+          float t = FLT_MAX;
+          if (sphere_isect(t, c3, q.w, c.r, c.prev_t, c.pn, self)) C.take(t, 0.0f, 0.0f, jj, lt);
+        }
+        __syncwarp();
+      }
+    }
+    __syncwarp();
+    bnd = bound_rel(G.min4(C.m), kRelTri);
+  }
+  w.branch = w.it;
+  if (G.lane) w.branch = w.leaf = w.prim = 0;  // the group's work, counted once
+  // merge the lanes' candidates
+  WidePass r;
+  const float m = G.min4(C.m);
+  const bool mine = C.m == m && m < FLT_MAX;
+  const unsigned holders = G.vote(mine);
+  const float second = G.min4(mine ? C.m2 : C.m);
+  // a single candidate below its box's entry e is hidden only by another
+  // primitive nearer than e (all tested: e lies below the pruning bound)
+  const bool single = !C.tie && (holders & (holders - 1)) == 0;
+  bool viol = below_entry(C.m, C.e) || C.tie_viol;
+  if (viol && single) viol = !(second >= C.e) || !(C.e < bound_rel(m, kRelTri));
+  r.viol = G.vote(mine && viol) != 0;
+  r.defer = G.vote(mine && (viol || !single)) != 0;
+  r.winner = G.shift + (holders ? __ffs(holders) - 1 : 0);
+  return r;
+}
+
+// The ray of lane `src`, whose record that lane holds in (a, b), for its
+// whole group.
+__device__ __forceinline__ Ctx2 group_ctx2(const float4 &a, const float4 &b, int src,
+                                           float keps) {
+  constexpr unsigned kAll = 0xffffffffu;
+  const float4 qa = make_float4(__shfl_sync(kAll, a.x, src), __shfl_sync(kAll, a.y, src),
+                                __shfl_sync(kAll, a.z, src), __shfl_sync(kAll, a.w, src));
+  const float4 qb = make_float4(__shfl_sync(kAll, b.x, src), __shfl_sync(kAll, b.y, src),
+                                __shfl_sync(kAll, b.z, src), __shfl_sync(kAll, b.w, src));
+  Ctx2 c;
+  c.r = ray_of(qa, qb);
+  c.prev_prim = __float_as_uint(qa.w);
+  c.prev_t = qb.w;
+  c.pn[0] = c.pn[1] = c.pn[2] = 0.0f;
+  c.keps = keps;
+  return c;
+}
+
+// A group's result on its way to the thread that stores it.
+struct WideSlot {
+  float t, u, v;
+  uint32_t j, state;  // state 0: final, 1: replay the tie at t, 3: the full walk
+};
+
+// The first pass of a block's 32 rays, 8 per warp; the first warp stores
+// them once all four are done, with its 32 lanes (a sphere's angles take
+// double-precision functions).
+// Bound by instruction issue: 58 to 65 % of issue slots busy, 20 to 25 of
+// 32 lanes active, DRAM idle.  131,072 triangles, 512^2 rays: 305 -> 164 us;
+// 1,000,003 triangles, 1280 x 720: 795 -> 437 us; 2,050 triangles, 96 x 64:
+// 56 -> 22 us (against the two-child walk).  Tried and slower: exchanges
+// within diverged groups (sub-warp masks, 511 us on the second), four rounds
+// of 8 rays per warp (935 us: the longest rays end the launch), pushing all
+// but the nearest child unsorted (500 us), 8 to 12 blocks per SM by launch
+// bounds (482 to 520 us: spills).
+template <int KIND>
+__global__ void __launch_bounds__(128)
+trace_wide_kernel(const WideRec *__restrict__ wide, uint32_t wide_cap,
+                  const Node2 *__restrict__ nodes, const float4 *__restrict__ prims,
+                  const uint32_t *__restrict__ sidx, const srt_ray *__restrict__ rays, size_t n,
+                  srt_hit *__restrict__ hits, const SceneInfo *__restrict__ scene,
+                  const float *__restrict__ prev_normals, float *__restrict__ normal_out,
+                  unsigned long long *__restrict__ stats, Deferred *__restrict__ dlist,
+                  uint32_t *__restrict__ dcount, uint32_t max_iter, uint32_t *__restrict__ err,
+                  const uint32_t *__restrict__ order) {
+  __shared__ uint2 s_stk[32][kWideStack];
+  __shared__ WideSlot s_res[32];
+  if (scene->nbranches > wide_cap) return;  // trace_node2_kernel traces the rays
+  const int lane = (int)(threadIdx.x & 31u), group = (int)(threadIdx.x >> 2);
+  const Group G;
+  // each warp holds its block's 32 rays, one per lane
+  const size_t base = (size_t)blockIdx.x * 32, k = base + (size_t)lane;
+  const bool have = k < n;
+  size_t i = 0;
+  float4 ra = make_float4(0.f, 0.f, 0.f, 0.f), rb = ra;
+  if (have) {
+    i = order ? (size_t)__ldg(&order[k]) : k;
+    const float4 *r4 = reinterpret_cast<const float4 *>(rays + i);
+    ra = __ldg(r4);
+    rb = __ldg(r4 + 1);
+  }
+  {
+    const WideTree<KIND> T = {wide, nodes, prims, sidx, scene->irregular != 0};
+    Ctx2 c = group_ctx2(ra, rb, group, scene->keps);
+    const size_t gi = (size_t)__shfl_sync(0xffffffffu, (unsigned long long)i, group);
+    const bool live = base + (size_t)group < n;
+    if (KIND == SRT_SPHERES && live && prev_normals && c.prev_prim != kNone) {
+      c.pn[0] = prev_normals[3 * gi];
+      c.pn[1] = prev_normals[3 * gi + 1];
+      c.pn[2] = prev_normals[3 * gi + 2];
+    }
+    Cand C;
+    Work w;
+    const WidePass p = pass1_wide<KIND>(T, G, c, 0u, live, s_stk[group], C, w, max_iter);
+    if (live && lane == p.winner) {
+      if (w.fail) atomicOr(err, kErrIter);
+      const uint32_t state = !w.fail && p.defer ? (p.viol ? 3u : 1u) : 0u;
+      s_res[group] = WideSlot{C.m, C.u, C.v, C.j, state};
+    }
+    add_stats(stats, w, 0);
+  }
+  // the other warps only arrive
+  if (threadIdx.x >= 32) {
+    asm volatile("bar.arrive 1, 128;" ::: "memory");
+    return;
+  }
+  asm volatile("bar.sync 1, 128;" ::: "memory");
+  if (!have) return;
+  const WideSlot s = s_res[lane];
+  if (s.state) {
+    const uint32_t q = atomicAdd(dcount, 1u);
+    dlist[q] = Deferred{(uint32_t)i, s.state >> 1, (double)s.t};
+    return;
+  }
+  Best b;
+  b.t = s.t;
+  b.u = s.u;
+  b.v = s.v;
+  b.j = s.j;
+  if (s.j != kNone)
+    b.prim = KIND == SRT_TRIANGLES ? __float_as_uint(__ldg(&prims[3 * (size_t)s.j].w))
+                                   : __ldg(&sidx[s.j]);
+  Ctx2 c;
+  if (KIND == SRT_SPHERES) c.r = ray_of(ra, rb);
+  store_node2<KIND>(i, b, c, prims, hits, normal_out);
+}
+
+// Whether n rays take the wide walk: always below kWideRays, where one
+// thread per ray cannot fill the GPU and its longest rays (a silhouette's
+// pass 200 nodes and 600 primitives where the mean is 14 and 11) end the
+// launch; with more, only triangles in trees that are not small -- enough
+// rays hide the chains, and a two-child node costs fewer instructions per
+// ray.  Measured, wide / two-child, us:
+//   spheres       100,000: 64^2 rays 56 / 168, 512^2 205 / 247, 1024^2 572 / 536
+//   spheres    12,000,000: 64^2 84 / 290, 512^2 433 / 555, 1400^2 3289 / 3247
+//   triangles       2,000: 64^2 26 / 48, 512^2 76 / 81, 1024^2 227 / 188
+//   triangles     100,000: 64^2 73 / 137, 512^2 177 / 309, 1400^2 707 / 805
+//   triangles   2,000,000: 64^2 118 / 215, 512^2 408 / 981, 1400^2 1217 / 1836
+constexpr size_t kWideRays = (size_t)1 << 19;
+constexpr size_t kWideTriangles = (size_t)1 << 15;
+bool takes_wide(const srt_accel *a, size_t n) {
+  return n < kWideRays || (a->kind == SRT_TRIANGLES && a->n >= kWideTriangles);
+}
+
 // Rays of a first-pass kernel: with `next` (a zeroed counter), persistent
 // warps take 32 consecutive rays at a time until all n are done, so every SM
 // stays busy to the end whatever the rays cost; without it, one thread per
@@ -851,7 +1239,8 @@ trace_node2_kernel(const Node2 *__restrict__ nodes, const float4 *__restrict__ p
                    unsigned long long *__restrict__ stats, Deferred *__restrict__ dlist,
                    uint32_t *__restrict__ dcount, uint32_t max_iter,
                    uint32_t *__restrict__ err, const uint32_t *__restrict__ order,
-                   uint32_t *__restrict__ next = nullptr) {
+                   uint32_t *__restrict__ next = nullptr, uint32_t wide_cap = 0) {
+  if (wide_cap && scene->nbranches <= wide_cap) return;  // trace_wide_kernel traced the rays
   for_each_ray(n, next, [&](size_t k) {
     const size_t i = order ? (size_t)__ldg(&order[k]) : k;  // ray of this thread
     const Ctx2 c = make_ctx2<KIND>(rays, i, scene, prev_normals);
@@ -1365,6 +1754,21 @@ int resident_blocks(const void *fn, int block) {
   return nb;
 }
 
+// The first pass over the wide nodes.
+static void launch_wide(srt_accel *a, const srt_ray *rays, size_t n, srt_hit *hits,
+                        const float *prev_normals, float *normal_out, unsigned long long *stats,
+                        Deferred *dlist, uint32_t *dcount, uint32_t max_iter,
+                        const uint32_t *order) {
+  srt_ctx *ctx = a->ctx;
+  const auto kern = a->kind == SRT_TRIANGLES ? trace_wide_kernel<SRT_TRIANGLES>
+                                             : trace_wide_kernel<SRT_SPHERES>;
+  kern<<<(unsigned)((n + 31) / 32), 128, 0, ctx->stream>>>(
+      a->wide.as<WideRec>(), a->wide_cap, a->nodes.as<Node2>(), a->prims.as<float4>(),
+      a->indices.as<uint32_t>(), rays, n, hits, a->scene.as<SceneInfo>(), prev_normals,
+      normal_out, stats, dlist, dcount, max_iter, ctx->d_err, order);
+  ctx->launches++;
+}
+
 srt_status launch_trace(srt_accel *a, const srt_ray *rays, size_t n, srt_hit *hits,
                         const float *prev_normals, uint32_t *subface,
                         const float *vscalar, float *scalar_out, float *normal_out,
@@ -1418,13 +1822,25 @@ srt_status launch_trace(srt_accel *a, const srt_ray *rays, size_t n, srt_hit *hi
       const float4 *pr = a->prims.as<float4>();
       const uint32_t *ix = a->indices.as<uint32_t>();
       const bool tri = a->kind == SRT_TRIANGLES;
-      const auto kern = tri ? (single ? trace_node2_kernel<SRT_TRIANGLES, true>
-                                      : trace_node2_kernel<SRT_TRIANGLES, false>)
-                            : (single ? trace_node2_kernel<SRT_SPHERES, true>
-                                      : trace_node2_kernel<SRT_SPHERES, false>);
-      kern<<<fgrid((const void *)kern), block, 0, st>>>(
-          nd, pr, ix, rays, n, hits, scene, pn, normal_out, stats, dlist, dcount, max_iter,
-          ctx->d_err, order, next);
+      // a caller's cap counts the two-child walk's steps, and a full-grid
+      // launch is that kernel's; a tree that may have more branches than wide
+      // nodes gets both kernels, each leaving the rays to the other by the
+      // branch count
+      const bool wide =
+          !single && !max_iter_cap && !(flags & SRT_TRACE_GRID) && takes_wide(a, n);
+      if (wide)
+        launch_wide(a, rays, n, hits, pn, normal_out, stats, dlist, dcount, max_iter, order);
+      if (!wide || !a->wide_all) {
+        const auto kern = tri ? (single ? trace_node2_kernel<SRT_TRIANGLES, true>
+                                        : trace_node2_kernel<SRT_TRIANGLES, false>)
+                              : (single ? trace_node2_kernel<SRT_SPHERES, true>
+                                        : trace_node2_kernel<SRT_SPHERES, false>);
+        kern<<<fgrid((const void *)kern), block, 0, st>>>(
+            nd, pr, ix, rays, n, hits, scene, pn, normal_out, stats, dlist, dcount, max_iter,
+            ctx->d_err, order, next, wide ? a->wide_cap : 0);
+      } else {
+        ctx->launches--;
+      }
       if (!single) {
         const auto res = tri ? resolve_node2_kernel<SRT_TRIANGLES>
                              : resolve_node2_kernel<SRT_SPHERES>;
@@ -2314,9 +2730,14 @@ extern "C" SRT_API srt_status srt_trace_closest_noalloc(srt_accel *a, const srt_
   switch (a->kind) {
     case SRT_TRIANGLES: {
       const Node2 *nd = a->nodes.as<Node2>();
-      trace_node2_kernel<SRT_TRIANGLES, false><<<grid, block, 0, st>>>(
-          nd, pr, ix, rays, n, hits, scene, nullptr, nullptr, nullptr, dlist, dcount, max_iter,
-          ctx->d_err, nullptr);
+      launch_wide(a, rays, n, hits, nullptr, nullptr, nullptr, dlist, dcount, max_iter, nullptr);
+      if (!a->wide_all) {
+        trace_node2_kernel<SRT_TRIANGLES, false><<<grid, block, 0, st>>>(
+            nd, pr, ix, rays, n, hits, scene, nullptr, nullptr, nullptr, dlist, dcount, max_iter,
+            ctx->d_err, nullptr, nullptr, a->wide_cap);
+        ctx->launches++;
+      }
+      ctx->launches--;
       resolve_node2_kernel<SRT_TRIANGLES><<<rgrid, block, 0, st>>>(
           nd, pr, ix, rays, hits, scene, nullptr, nullptr, nullptr, dlist, dcount, max_iter,
           ctx->d_err);
@@ -2324,9 +2745,14 @@ extern "C" SRT_API srt_status srt_trace_closest_noalloc(srt_accel *a, const srt_
     }
     case SRT_SPHERES: {
       const Node2 *nd = a->nodes.as<Node2>();
-      trace_node2_kernel<SRT_SPHERES, false><<<grid, block, 0, st>>>(
-          nd, pr, ix, rays, n, hits, scene, nullptr, nullptr, nullptr, dlist, dcount, max_iter,
-          ctx->d_err, nullptr);
+      launch_wide(a, rays, n, hits, nullptr, nullptr, nullptr, dlist, dcount, max_iter, nullptr);
+      if (!a->wide_all) {
+        trace_node2_kernel<SRT_SPHERES, false><<<grid, block, 0, st>>>(
+            nd, pr, ix, rays, n, hits, scene, nullptr, nullptr, nullptr, dlist, dcount, max_iter,
+            ctx->d_err, nullptr, nullptr, a->wide_cap);
+        ctx->launches++;
+      }
+      ctx->launches--;
       resolve_node2_kernel<SRT_SPHERES><<<rgrid, block, 0, st>>>(
           nd, pr, ix, rays, hits, scene, nullptr, nullptr, nullptr, dlist, dcount, max_iter,
           ctx->d_err);
