@@ -1266,6 +1266,134 @@ trace_node2_kernel(const Node2 *__restrict__ nodes, const float4 *__restrict__ p
   });
 }
 
+// --------------------------------------------------------------- warp walks
+// The reference-order walks with a warp per ray, for the rays the first pass
+// leaves open.  They are few (two hundred of 4 M, typically) and their walks
+// long, so one thread each is a chain of hundreds of nodes and a thousand
+// primitives that ends the launch; here a leaf's primitives are tested by 32
+// lanes at once and every branch is uniform.  16,777,216 spheres, 2048^2
+// rays: 1.34 -> 0.22 ms per launch; a batch of 64 scenes: 270 -> 57 us.  Above kWarpRays open rays (scenes of
+// duplicated primitives) a thread per ray has the better throughput.
+constexpr uint32_t kWarpRays = 1u << 16;
+// Tetrahedra: a leaf holds five at most, so a warp per ray pays only while
+// the rays do not fill the GPU (65,536 open rays of a 64^3 x 5 mesh: 635 us
+// by warps, 255 us by threads).
+constexpr uint32_t kWarpTetRays = 1u << 13;
+
+// ref_walk2 (WINDOW false: running distance from t0, boxes pruned by it) or
+// window_walk2 (WINDOW true: boxes entered before bnd), in every lane's b.
+// stk: the warp's kStack entries.
+template <int KIND, bool WINDOW>
+__device__ void walk2_warp(const Node2 *__restrict__ nodes, const float4 *__restrict__ prims,
+                           const uint32_t *__restrict__ sidx, const Ctx2 &c, float bnd, float t0,
+                           uint2 *stk, Best &b, Work &w, uint32_t max_iter, uint32_t root) {
+  constexpr unsigned kAll = 0xffffffffu;
+  const uint32_t lane = threadIdx.x & 31u;
+  b = Best();
+  float t = t0;
+  int sp = 0;
+  __syncwarp();
+  if (lane == 0) stk[0] = make_uint2(root, 0u);
+  __syncwarp();
+  while (sp >= 0) {
+    if (++w.it > max_iter) { w.fail = true; break; }
+    const uint2 e = stk[sp--];
+    __syncwarp();  // read by every lane before a push overwrites it
+    if (e.y == 0) {
+      if (lane == 0) w.branch++;
+      const float4 *np = reinterpret_cast<const float4 *>(nodes + e.x);
+      const float4 a = __ldg(np), bb = __ldg(np + 1), cc = __ldg(np + 2);
+      const uint4 d = __ldg(reinterpret_cast<const uint4 *>(np + 3));
+      const float lim = WINDOW ? bnd : t;
+      const bool h0 = ray_aabb<true>(lim, a.x, a.y, a.z, a.w, bb.x, bb.y, c.r);
+      const bool h1 = ray_aabb<true>(lim, bb.z, bb.w, cc.x, cc.y, cc.z, cc.w, c.r);
+      if (h0 || h1) {
+        const int nearc = c.r.sgn[d.z >> 30];
+        const uint2 c0 = make_uint2(d.x, d.z & kCountMask), c1 = make_uint2(d.y, d.w & kCountMask);
+        if (sp + 2 >= kStack) { w.fail = true; break; }
+        if (nearc ? h0 : h1) stk[++sp] = nearc ? c0 : c1;  // far
+        if (nearc ? h1 : h0) stk[++sp] = nearc ? c1 : c0;  // near
+      }
+      __syncwarp();
+      continue;
+    }
+    if (lane == 0) {
+      w.leaf++;
+      w.prim += e.y;
+    }
+    for (uint32_t j0 = e.x; j0 < e.x + e.y; j0 += 32) {
+      const uint32_t j = j0 + lane;
+      float tj = FLT_MAX, u = 0.0f, v = 0.0f;
+      uint32_t f = kNone;
+      bool hit = false;
+      if (j < e.x + e.y) hit = cand2<KIND>(prims, sidx, j, c, t, tj, u, v, f);
+      const unsigned hits = __ballot_sync(kAll, hit);
+      if (!hits) continue;
+      // one after the other, a triangle at the running distance replaces it
+      // and a sphere does not: the last or first of the nearest
+      const uint32_t key = hit ? __float_as_uint(tj + 0.0f) : 0xffffffffu;
+      const uint32_t least = __reduce_min_sync(kAll, key);
+      const unsigned best = __ballot_sync(kAll, hit && key == least);
+      const int src = KIND == SRT_TRIANGLES ? 31 - __clz(best) : __ffs(best) - 1;
+      b.t = t = __shfl_sync(kAll, tj, src);
+      b.u = __shfl_sync(kAll, u, src);
+      b.v = __shfl_sync(kAll, v, src);
+      b.prim = __shfl_sync(kAll, f, src);
+      b.j = j0 + (uint32_t)src;
+    }
+  }
+  if (!WINDOW && b.prim == kNone) b.t = FLT_MAX;
+}
+
+// An open ray's replay by its warp: ref_walk2_from, or window_walk2 at m.
+template <int KIND>
+__device__ __forceinline__ void replay2_warp(const Node2 *__restrict__ nodes,
+                                             const float4 *__restrict__ prims,
+                                             const uint32_t *__restrict__ sidx, const Ctx2 &c,
+                                             bool full, float m, uint2 *stk, Best &b, Work &w,
+                                             uint32_t max_iter, uint32_t root) {
+  if (full) {
+    walk2_warp<KIND, false>(nodes, prims, sidx, c, 0.0f, bound_rel(m, kRelTri), stk, b, w,
+                            max_iter, root);
+    if (b.prim != kNone || w.fail) return;
+    w.it = 0;
+    walk2_warp<KIND, false>(nodes, prims, sidx, c, 0.0f, FLT_MAX, stk, b, w, max_iter, root);
+  } else {
+    const float t0 = (KIND == SRT_TRIANGLES) ? m : nextafterf(m, FLT_MAX);
+    walk2_warp<KIND, true>(nodes, prims, sidx, c, bound_rel(m, kRelTri), t0, stk, b, w, max_iter,
+                           root);
+  }
+}
+
+// The same with a thread per ray.
+template <int KIND>
+__device__ __forceinline__ void replay2(const Node2 *__restrict__ nodes,
+                                        const float4 *__restrict__ prims,
+                                        const uint32_t *__restrict__ sidx, const Ctx2 &c,
+                                        bool full, float m, Best &b, Work &w, uint32_t max_iter,
+                                        uint32_t root) {
+  if (full) {
+    ref_walk2_from<KIND>(nodes, prims, sidx, c, b, w, max_iter, m, root);
+  } else {
+    // triangles keep the last candidate at m (t <= current), spheres the
+    // first (t < current)
+    const float t0 = (KIND == SRT_TRIANGLES) ? m : nextafterf(m, FLT_MAX);
+    window_walk2<KIND>(nodes, prims, sidx, c, bound_rel(m, kRelTri), t0, b, w, max_iter, root);
+  }
+}
+
+// The open rays: body(k, warp) for item k, by a warp (up to `most` of them)
+// or by a thread.
+template <typename Body>
+__device__ __forceinline__ void for_each_open(uint32_t cnt, uint32_t most, const Body &body) {
+  const uint32_t thread = blockIdx.x * blockDim.x + threadIdx.x, threads = gridDim.x * blockDim.x;
+  if (cnt <= most) {
+    for (uint32_t k = thread >> 5; k < cnt; k += threads >> 5) body(k, true);
+  } else {
+    for (uint32_t k = thread; k < cnt; k += threads) body(k, false);
+  }
+}
+
 template <int KIND>
 __global__ void __launch_bounds__(128)
 resolve_node2_kernel(const Node2 *__restrict__ nodes, const float4 *__restrict__ prims,
@@ -1275,26 +1403,23 @@ resolve_node2_kernel(const Node2 *__restrict__ nodes, const float4 *__restrict__
                      float *__restrict__ normal_out, unsigned long long *__restrict__ stats,
                      const Deferred *__restrict__ dlist, const uint32_t *__restrict__ dcount,
                      uint32_t max_iter, uint32_t *__restrict__ err) {
-  const uint32_t cnt = *dcount;
-  for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < cnt;
-       k += gridDim.x * blockDim.x) {
+  __shared__ uint2 s_stk[4][kStack];
+  for_each_open(*dcount, kWarpRays, [&](uint32_t k, bool warp) {
     const Deferred dfr = dlist[k];
     const Ctx2 c = make_ctx2<KIND>(rays, dfr.ray, scene, prev_normals);
     Work w;
     Best b;
-    if (dfr.full) {
-      ref_walk2_from<KIND>(nodes, prims, sidx, c, b, w, max_iter, (float)dfr.m);
+    if (warp) {
+      replay2_warp<KIND>(nodes, prims, sidx, c, dfr.full, (float)dfr.m, s_stk[threadIdx.x >> 5],
+                         b, w, max_iter, 0u);
+      if (threadIdx.x & 31u) return;
     } else {
-      // triangles keep the last candidate at m (t <= current), spheres the
-      // first (t < current)
-      const float m = (float)dfr.m;
-      const float t0 = (KIND == SRT_TRIANGLES) ? m : nextafterf(m, FLT_MAX);
-      window_walk2<KIND>(nodes, prims, sidx, c, bound_rel(m, kRelTri), t0, b, w, max_iter);
+      replay2<KIND>(nodes, prims, sidx, c, dfr.full, (float)dfr.m, b, w, max_iter, 0u);
     }
     if (w.fail) atomicOr(err, kErrIter);
     add_stats(stats, w, dfr.full);
     store_node2<KIND>(dfr.ray, b, c, prims, hits, normal_out);
-  }
+  });
 }
 
 // ---- tetrahedra (own-box nodes, FP64 entry distance)
@@ -1346,31 +1471,59 @@ __device__ __forceinline__ void take_tet(Best &b, double te, double e1, double e
 // The reference's walk (render/render_accel_tetra.cc:2200) with the
 // running distance starting at t0 or, with WINDOW, the reference order
 // through boxes entered before `bnd` keeping only candidates at most `whi`
-// away.
+// away.  The reference pops a node and then tests its box; here a branch
+// tests both children's, half as many dependent loads, and a popped entry
+// compares its entry distance with the running distance, which is all of
+// that test that can have changed.  Steps count as the reference's pops: two
+// per entered branch.
 template <bool WINDOW, typename P = float4>
 __device__ void walkT(const NodeT *__restrict__ nodes, const P *__restrict__ prims,
                       const uint32_t *__restrict__ sidx, const CtxT &c, float bnd,
                       double whi, Best &b, Work &w, uint32_t max_iter, float t0 = FLT_MAX) {
   b = Best();
   float t = t0;
-  uint32_t stk[kStack];
-  int sp = 0;
-  stk[0] = 0u;
+  uint2 stk[kStack];  // (ref, meta)
+  float stt[kStack];  // entry distance
+  int sp = -1;
+  {
+    const float4 *np = reinterpret_cast<const float4 *>(nodes);
+    const float4 a = __ldg(np), bb = __ldg(np + 1);
+    float te;
+    w.it++;
+    if (ray_aabb_t<false>(WINDOW ? bnd : t, a.x, a.y, a.z, bb.x, bb.y, bb.z, c.r, te)) {
+      stk[0] = make_uint2(__float_as_uint(bb.w), __float_as_uint(a.w));
+      stt[0] = te;
+      sp = 0;
+    }
+  }
   while (true) {
     uint32_t lref = 0, lcnt = 0;
     while (sp >= 0) {
-      if (++w.it > max_iter) { w.fail = true; sp = -1; break; }
-      const uint32_t ni = stk[sp--];
-      const float4 *np = reinterpret_cast<const float4 *>(nodes + ni);
-      const float4 a = __ldg(np), bb = __ldg(np + 1);
-      const uint32_t meta = __float_as_uint(a.w), ref = __float_as_uint(bb.w);
+      if (w.it > max_iter) { w.fail = true; sp = -1; break; }
+      const uint2 e = stk[sp];
+      const float et = stt[sp--];
+      if (!(et <= (WINDOW ? bnd : t))) continue;
+      if (e.y & kLeafBit) { lref = e.x; lcnt = e.y & kCountMask; break; }
       w.branch++;
-      if (!ray_aabb<false>(WINDOW ? bnd : t, a.x, a.y, a.z, bb.x, bb.y, bb.z, c.r)) continue;
-      if (meta & kLeafBit) { lref = ref; lcnt = meta & kCountMask; break; }
-      const int nearc = c.r.sgn[meta & 3u], farc = 1 - nearc;
+      w.it += 2;
+      const float4 *cp = reinterpret_cast<const float4 *>(nodes + e.x);
+      const float4 a0 = __ldg(cp), b0 = __ldg(cp + 1), a1 = __ldg(cp + 2), b1 = __ldg(cp + 3);
+      float t0c, t1c;
+      const float lim = WINDOW ? bnd : t;
+      const bool h0 = ray_aabb_t<false>(lim, a0.x, a0.y, a0.z, b0.x, b0.y, b0.z, c.r, t0c);
+      const bool h1 = ray_aabb_t<false>(lim, a1.x, a1.y, a1.z, b1.x, b1.y, b1.z, c.r, t1c);
+      const uint2 e0 = make_uint2(__float_as_uint(b0.w), __float_as_uint(a0.w)),
+                  e1 = make_uint2(__float_as_uint(b1.w), __float_as_uint(a1.w));
+      const bool near1 = c.r.sgn[e.y & 3u] != 0;
       if (sp + 2 >= kStack) { w.fail = true; sp = -1; break; }
-      stk[++sp] = ref + (uint32_t)farc;
-      stk[++sp] = ref + (uint32_t)nearc;
+      if (near1 ? h0 : h1) {  // far
+        stk[++sp] = near1 ? e0 : e1;
+        stt[sp] = near1 ? t0c : t1c;
+      }
+      if (near1 ? h1 : h0) {  // near
+        stk[++sp] = near1 ? e1 : e0;
+        stt[sp] = near1 ? t1c : t0c;
+      }
     }
     if (lcnt == 0) break;
     w.leaf++;
@@ -1407,6 +1560,124 @@ __device__ __forceinline__ void walkT_from(const NodeT *__restrict__ nodes,
   if (b.prim != kNone || w.fail) return;
   w.it = 0;
   walkT<false, P>(nodes, prims, sidx, c, 0.0f, 0.0, b, w, max_iter);
+}
+
+// walkT with a warp per ray: the lanes test a leaf's tetrahedra side by side,
+// then those hit are taken in order by walkT's rule (the running distance is
+// rounded to float after each).  stk: the warp's kStack entries.
+template <bool WINDOW, typename P>
+__device__ void walkT_warp(const NodeT *__restrict__ nodes, const P *__restrict__ prims,
+                           const uint32_t *__restrict__ sidx, const CtxT &c, float bnd, double whi,
+                           uint4 *stk, Best &b, Work &w, uint32_t max_iter,
+                           float t0 = FLT_MAX) {
+  constexpr unsigned kAll = 0xffffffffu;
+  const uint32_t lane = threadIdx.x & 31u;
+  b = Best();
+  float t = t0;
+  int sp = -1;
+  __syncwarp();
+  {
+    const float4 *np = reinterpret_cast<const float4 *>(nodes);
+    const float4 a = __ldg(np), bb = __ldg(np + 1);
+    float te;
+    w.it++;
+    if (ray_aabb_t<false>(WINDOW ? bnd : t, a.x, a.y, a.z, bb.x, bb.y, bb.z, c.r, te)) {
+      sp = 0;
+      if (lane == 0)
+        stk[0] = make_uint4(__float_as_uint(bb.w), __float_as_uint(a.w), __float_as_uint(te), 0u);
+    }
+  }
+  __syncwarp();
+  while (sp >= 0) {
+    if (w.it > max_iter) { w.fail = true; break; }
+    const uint4 e = stk[sp--];
+    __syncwarp();  // read by every lane before a push overwrites it
+    if (!(__uint_as_float(e.z) <= (WINDOW ? bnd : t))) continue;
+    if (!(e.y & kLeafBit)) {
+      if (lane == 0) w.branch++;
+      w.it += 2;
+      const float4 *cp = reinterpret_cast<const float4 *>(nodes + e.x);
+      const float4 a0 = __ldg(cp), b0 = __ldg(cp + 1), a1 = __ldg(cp + 2), b1 = __ldg(cp + 3);
+      float t0c, t1c;
+      const float lim = WINDOW ? bnd : t;
+      const bool h0 = ray_aabb_t<false>(lim, a0.x, a0.y, a0.z, b0.x, b0.y, b0.z, c.r, t0c);
+      const bool h1 = ray_aabb_t<false>(lim, a1.x, a1.y, a1.z, b1.x, b1.y, b1.z, c.r, t1c);
+      const uint4 e0 = make_uint4(__float_as_uint(b0.w), __float_as_uint(a0.w),
+                                  __float_as_uint(t0c), 0u),
+                  e1 = make_uint4(__float_as_uint(b1.w), __float_as_uint(a1.w),
+                                  __float_as_uint(t1c), 0u);
+      const bool near1 = c.r.sgn[e.y & 3u] != 0;
+      if (sp + 2 >= kStack) { w.fail = true; break; }
+      if (near1 ? h0 : h1) stk[++sp] = near1 ? e0 : e1;  // far
+      if (near1 ? h1 : h0) stk[++sp] = near1 ? e1 : e0;  // near
+      __syncwarp();
+      continue;
+    }
+    const uint32_t cnt = e.y & kCountMask;
+    if (lane == 0) {
+      w.leaf++;
+      w.prim += cnt;
+    }
+    for (uint32_t j0 = e.x; j0 < e.x + cnt; j0 += 32) {
+      const uint32_t j = j0 + lane;
+      uint32_t f = kNone;
+      int ef = 0;
+      double e1 = 0.0, e2 = 0.0, ul1 = 0.0, te = DBL_MAX;
+      bool hit = false;
+      if (j < e.x + cnt) hit = candT(prims, sidx, j, c, (double)t, f, ef, e1, e2, ul1, te);
+      if (WINDOW) hit = hit && te <= whi;
+      unsigned hits = __ballot_sync(kAll, hit && te < (double)t);
+      int src = -1;
+      while (hits) {
+        const int l = __ffs(hits) - 1;
+        hits &= hits - 1;
+        const double tl = __shfl_sync(kAll, te, l);
+        if (tl < (double)t) {
+          t = (float)tl;
+          src = l;
+        }
+      }
+      if (src >= 0)
+        take_tet(b, __shfl_sync(kAll, te, src), __shfl_sync(kAll, e1, src),
+                 __shfl_sync(kAll, e2, src), __shfl_sync(kAll, ul1, src),
+                 __shfl_sync(kAll, f, src), __shfl_sync(kAll, ef, src));
+    }
+  }
+}
+
+// An open ray's replay: the reference's walk from the pass's bound (full) or
+// the reference order through the window at m, by a warp (with its stack) or
+// by one thread.
+template <typename P>
+__device__ __forceinline__ void replayT_warp(const NodeT *__restrict__ nodes,
+                                             const P *__restrict__ prims,
+                                             const uint32_t *__restrict__ sidx, const CtxT &c,
+                                             bool full, double m, uint4 *stk, Best &b, Work &w,
+                                             uint32_t max_iter) {
+  if (full) {
+    walkT_warp<false>(nodes, prims, sidx, c, 0.0f, 0.0, stk, b, w, max_iter,
+                      bound_rel((float)m, kRelTet));
+    if (b.prim != kNone || w.fail) return;
+    w.it = 0;
+    walkT_warp<false>(nodes, prims, sidx, c, 0.0f, 0.0, stk, b, w, max_iter);
+  } else {
+    const double whi = window_hi(m);
+    walkT_warp<true>(nodes, prims, sidx, c, bound_rel((float)whi, kRelTet), whi, stk, b, w,
+                     max_iter);
+  }
+}
+template <typename P>
+__device__ __forceinline__ void replayT(const NodeT *__restrict__ nodes,
+                                        const P *__restrict__ prims,
+                                        const uint32_t *__restrict__ sidx, const CtxT &c,
+                                        bool full, double m, Best &b, Work &w,
+                                        uint32_t max_iter) {
+  if (full) {
+    walkT_from(nodes, prims, sidx, c, b, w, max_iter, m);
+  } else {
+    const double whi = window_hi(m);
+    walkT<true>(nodes, prims, sidx, c, bound_rel((float)whi, kRelTet), whi, b, w, max_iter);
+  }
 }
 
 __device__ __forceinline__ void store_tet(size_t i, const Best &b,
@@ -1628,24 +1899,23 @@ resolve_tet_kernel(const NodeT *__restrict__ nodes, const P *__restrict__ prims,
                    float *__restrict__ scalar_out, unsigned long long *__restrict__ stats,
                    const Deferred *__restrict__ dlist, const uint32_t *__restrict__ dcount,
                    uint32_t max_iter, uint32_t *__restrict__ err) {
-  const uint32_t cnt = *dcount;
-  for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < cnt;
-       k += gridDim.x * blockDim.x) {
+  __shared__ uint4 s_stk[4][kStack];
+  for_each_open(*dcount, kWarpTetRays, [&](uint32_t k, bool warp) {
     const Deferred dfr = dlist[k];
     const CtxT c = make_ctxT(rays, dfr.ray);
     Work w;
     Best b;
-    if (dfr.full) {
-      walkT_from(nodes, prims, sidx, c, b, w, max_iter, dfr.m);
+    if (warp) {
+      replayT_warp(nodes, prims, sidx, c, dfr.full, dfr.m, s_stk[threadIdx.x >> 5], b, w,
+                   max_iter);
+      if (threadIdx.x & 31u) return;
     } else {
-      const double whi = window_hi(dfr.m);
-      walkT<true>(nodes, prims, sidx, c, bound_rel((float)whi, kRelTet), whi, b, w,
-                  max_iter);
+      replayT(nodes, prims, sidx, c, dfr.full, dfr.m, b, w, max_iter);
     }
     if (w.fail) atomicOr(err, kErrIter);
     add_stats(stats, w, dfr.full);
     store_tet(dfr.ray, b, hits, subface, faces, vscalar, scalar_out);
-  }
+  });
 }
 
 // --------------------------------------------------------------- batches
@@ -1709,9 +1979,8 @@ resolve_batch_kernel(const Node2 *__restrict__ nodes, const float4 *__restrict__
                      unsigned long long *__restrict__ stats,
                      const Deferred *__restrict__ dlist, const uint32_t *__restrict__ dcount,
                      uint32_t max_iter, uint32_t *__restrict__ err) {
-  const uint32_t cnt = *dcount;
-  for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < cnt;
-       k += gridDim.x * blockDim.x) {
+  __shared__ uint2 s_stk[4][kStack];
+  for_each_open(*dcount, kWarpRays, [&](uint32_t k, bool warp) {
     const Deferred dfr = dlist[k];
     const int sg = seg_of(roff, nseg, dfr.ray);
     Ctx2 c;
@@ -1721,18 +1990,18 @@ resolve_batch_kernel(const Node2 *__restrict__ nodes, const float4 *__restrict__
     const uint32_t root = __ldg(&roots[sg]);
     Work w;
     Best b;
-    if (dfr.full) {
-      ref_walk2_from<SRT_TRIANGLES>(nodes, prims, nullptr, c, b, w, max_iter, (float)dfr.m,
-                                    root);
+    if (warp) {
+      replay2_warp<SRT_TRIANGLES>(nodes, prims, nullptr, c, dfr.full, (float)dfr.m,
+                                  s_stk[threadIdx.x >> 5], b, w, max_iter, root);
+      if (threadIdx.x & 31u) return;
     } else {
-      const float m = (float)dfr.m;
-      window_walk2<SRT_TRIANGLES>(nodes, prims, nullptr, c, bound_rel(m, kRelTri), m, b, w,
-                                  max_iter, root);
+      replay2<SRT_TRIANGLES>(nodes, prims, nullptr, c, dfr.full, (float)dfr.m, b, w, max_iter,
+                             root);
     }
     if (w.fail) atomicOr(err, kErrIter);
     add_stats(stats, w, dfr.full);
     store_node2<SRT_TRIANGLES>(dfr.ray, b, c, prims, hits, nullptr);
-  }
+  });
 }
 
 }  // namespace
@@ -2139,8 +2408,7 @@ __device__ __forceinline__ bool elem_pass1(const SceneElem &e, const typename Ki
   }
 }
 
-// The replay of an inconclusive pass: the reference's walk from the pass's
-// bound (full) or the reference order through the window at m.
+// The replay of an inconclusive pass, by one thread or (stk) by a warp.
 template <int KIND>
 __device__ __forceinline__ void elem_replay(const SceneElem &e,
                                             const typename KindCtx<KIND>::T &c, Best &b,
@@ -2148,29 +2416,31 @@ __device__ __forceinline__ void elem_replay(const SceneElem &e,
   w.it = 0;
   if constexpr (KIND == SRT_TETRAHEDRA) {
     const NodeT *nodes = static_cast<const NodeT *>(e.nodes);
-    auto replay = [&](auto *prims) {
-      if (full) {
-        walkT_from(nodes, prims, e.sidx, c, b, w, max_iter, m);
-      } else {
-        const double whi = window_hi(m);
-        walkT<true>(nodes, prims, e.sidx, c, bound_rel((float)whi, kRelTet), whi, b, w,
-                    max_iter);
-      }
-    };
     if (e.aux & kTetAuxDouble)
-      replay(reinterpret_cast<const double2 *>(e.prims));
+      replayT(nodes, reinterpret_cast<const double2 *>(e.prims), e.sidx, c, full, m, b, w,
+              max_iter);
     else
-      replay(e.prims);
+      replayT(nodes, e.prims, e.sidx, c, full, m, b, w, max_iter);
   } else {
-    const Node2 *nodes = static_cast<const Node2 *>(e.nodes);
-    const float mf = (float)m;
-    if (full) {
-      ref_walk2_from<KIND>(nodes, e.prims, e.sidx, c, b, w, max_iter, mf);
-    } else {
-      const float t0 = (KIND == SRT_TRIANGLES) ? mf : nextafterf(mf, FLT_MAX);
-      window_walk2<KIND>(nodes, e.prims, e.sidx, c, bound_rel(mf, kRelTri), t0, b, w,
-                         max_iter);
-    }
+    replay2<KIND>(static_cast<const Node2 *>(e.nodes), e.prims, e.sidx, c, full, (float)m, b, w,
+                  max_iter, 0u);
+  }
+}
+template <int KIND>
+__device__ __forceinline__ void elem_replay_warp(const SceneElem &e,
+                                                 const typename KindCtx<KIND>::T &c, uint4 *stk,
+                                                 Best &b, Work &w, uint32_t max_iter, double m,
+                                                 bool full) {
+  if constexpr (KIND == SRT_TETRAHEDRA) {
+    const NodeT *nodes = static_cast<const NodeT *>(e.nodes);
+    if (e.aux & kTetAuxDouble)
+      replayT_warp(nodes, reinterpret_cast<const double2 *>(e.prims), e.sidx, c, full, m, stk, b,
+                   w, max_iter);
+    else
+      replayT_warp(nodes, e.prims, e.sidx, c, full, m, stk, b, w, max_iter);
+  } else {
+    replay2_warp<KIND>(static_cast<const Node2 *>(e.nodes), e.prims, e.sidx, c, full, (float)m,
+                       reinterpret_cast<uint2 *>(stk), b, w, max_iter, 0u);
   }
 }
 
@@ -2332,11 +2602,11 @@ scene_walk_kernel(SceneWork W, int phase) {
 template <int KIND>
 __global__ void __launch_bounds__(128)
 scene_resolve_kernel(SceneWork W, int phase) {
+  __shared__ uint4 s_stk[4][kStack];
   const uint32_t lo = *(volatile uint32_t *)&W.bounds[4 * phase + KIND];
   const uint32_t cnt = *(volatile uint32_t *)&W.counters[10 + 3 * phase + KIND];
   uint32_t c[4] = {0, 0, 0, 0};
-  for (uint32_t k = blockIdx.x * blockDim.x + threadIdx.x; k < cnt;
-       k += gridDim.x * blockDim.x) {
+  for_each_open(cnt, KIND == SRT_TETRAHEDRA ? kWarpTetRays : kWarpRays, [&](uint32_t k, bool warp) {
     const Deferred d = W.dlist[lo + k];
     uint32_t ray, slot;
     item_ray_slot(phase, d.ray, ray, slot);
@@ -2350,14 +2620,18 @@ scene_resolve_kernel(SceneWork W, int phase) {
     const auto ctx = elem_ctx<KIND>(W, ray, e_id, e, r0, prev_prim, prev_t, lo3, ld3);
     Best b;
     Work w;
-    elem_replay<KIND>(e, ctx, b, w, W.max_iter, d.m, d.full != 0);
+    if (warp)
+      elem_replay_warp<KIND>(e, ctx, s_stk[threadIdx.x >> 5], b, w, W.max_iter, d.m, d.full != 0);
+    else
+      elem_replay<KIND>(e, ctx, b, w, W.max_iter, d.m, d.full != 0);
     c[1] += w.branch;
     c[2] += w.leaf;
     c[3] += w.prim;
+    if (warp && (threadIdx.x & 31u)) return;
     if (w.fail) atomicOr(W.err, kErrIter);
     if constexpr (KIND == SRT_SPHERES) elem_sphere_uv(ctx, e, b);
     finish_item(W, phase, ray, cs, e_id, e, lo3, ld3, r0.o, b);
-  }
+  });
   if (W.stats) add_counts(W.stats, 1, c, 4);
 }
 
