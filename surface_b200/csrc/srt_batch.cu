@@ -75,19 +75,23 @@ srt_status upload_offsets(srt_batch *b) {
 
 // The traversal as tuned: the batch ray order (when sorting) and the trace.
 srt_status trace_tuned(srt_batch *b, int block, int R, int depth, int sort_bits) {
-  const uint32_t *order = nullptr;
-  if (sort_bits > 0) {
-    const size_t n = b->bt.nrays;
-    cudaError_t e;
+  const size_t n = b->bt.nrays;
+  cudaError_t e;
+  if (sort_bits == 0) {  // the scenes' rays in tiles of their rows
+    if ((e = b->rorder.ensure(n * 4)) != cudaSuccess) return cuda_status(e, "batch ray order");
+    srt_status s = raster_order(b->ctx, b->rays, n, b->bt.roff.as<uint32_t>(), b->bt.nseg,
+                                b->rorder.as<uint32_t>());
+    if (s != SRT_OK) return s;
+  } else {
     if ((e = b->rkey.ensure(n * 4 + 64)) != cudaSuccess ||
         (e = b->rorder.ensure(n * 4)) != cudaSuccess)
       return cuda_status(e, "batch ray order");
     srt_status s = batch_ray_order(b->ctx, b->rays, n, b->bt.roff.as<uint32_t>(), b->bt.nseg,
                                    sort_bits, b->rkey.as<uint32_t>(), b->rorder.as<uint32_t>());
     if (s != SRT_OK) return s;
-    order = b->rorder.as<uint32_t>();
   }
-  return launch_trace_batch(b->ctx, b->bt, b->rays, b->hits, block, R, nullptr, depth, order);
+  return launch_trace_batch(b->ctx, b->bt, b->rays, b->hits, block, R, nullptr, depth,
+                            b->rorder.as<uint32_t>());
 }
 
 srt_status build_and_trace(srt_batch *b, const uint32_t *h_foff) {

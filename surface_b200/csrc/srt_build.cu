@@ -501,9 +501,12 @@ __device__ uint32_t block_exclusive_scan(uint32_t (&x)[kScanItems]) {
   return r;
 }
 
+// (the scan and sort kernels return at once when *skip is set)
 __global__ void scan_tiles_kernel(const uint32_t *__restrict__ in,
                                   uint32_t *__restrict__ out, size_t n,
-                                  uint32_t *__restrict__ tile_sums) {
+                                  uint32_t *__restrict__ tile_sums,
+                                  const uint32_t *__restrict__ skip) {
+  if (skip && *skip) return;
   size_t base = (size_t)blockIdx.x * kScanTile + (size_t)threadIdx.x * kScanItems;
   uint32_t x[kScanItems];
 #pragma unroll
@@ -516,7 +519,9 @@ __global__ void scan_tiles_kernel(const uint32_t *__restrict__ in,
 }
 
 __global__ void scan_add_kernel(uint32_t *__restrict__ out, size_t n,
-                                const uint32_t *__restrict__ tile_off) {
+                                const uint32_t *__restrict__ tile_off,
+                                const uint32_t *__restrict__ skip) {
+  if (skip && *skip) return;
   uint32_t add = tile_off[blockIdx.x];
   size_t base = (size_t)blockIdx.x * kScanTile;
   for (int i = threadIdx.x; i < kScanTile; i += blockDim.x)
@@ -528,34 +533,35 @@ __global__ void scan_add_kernel(uint32_t *__restrict__ out, size_t n,
 // Exclusive scan of n uint32 (out may alias in); tile sums of each level go
 // to `scratch` (needs about n / 4095 + 4 words).
 static srt_status scan_levels(cudaStream_t st, const uint32_t *in, uint32_t *out,
-                              size_t n, uint32_t *scratch, uint64_t &launches) {
+                              size_t n, uint32_t *scratch, uint64_t &launches,
+                              const uint32_t *skip) {
   size_t tiles = (n + kScanTile - 1) / kScanTile;
   if (tiles <= 1) {
-    scan_tiles_kernel<<<1, kScanThreads, 0, st>>>(in, out, n, nullptr);
+    scan_tiles_kernel<<<1, kScanThreads, 0, st>>>(in, out, n, nullptr, skip);
     launches++;
     return cuda_status(cudaGetLastError(), "scan");
   }
   uint32_t *sums = scratch;
-  scan_tiles_kernel<<<(unsigned)tiles, kScanThreads, 0, st>>>(in, out, n, sums);
+  scan_tiles_kernel<<<(unsigned)tiles, kScanThreads, 0, st>>>(in, out, n, sums, skip);
   launches++;
   srt_status s = cuda_status(cudaGetLastError(), "scan tiles");
   if (s != SRT_OK) return s;
-  s = scan_levels(st, sums, sums, tiles, scratch + tiles, launches);
+  s = scan_levels(st, sums, sums, tiles, scratch + tiles, launches, skip);
   if (s != SRT_OK) return s;
-  scan_add_kernel<<<(unsigned)tiles, 256, 0, st>>>(out, n, sums);
+  scan_add_kernel<<<(unsigned)tiles, 256, 0, st>>>(out, n, sums, skip);
   launches++;
   return cuda_status(cudaGetLastError(), "scan add");
 }
 
 static srt_status exclusive_scan(srt_ctx *ctx, const uint32_t *in, uint32_t *out,
-                                 size_t n) {
+                                 size_t n, const uint32_t *skip = nullptr) {
   size_t need = 64;
   for (size_t t = (n + kScanTile - 1) / kScanTile; t > 1;
        t = (t + kScanTile - 1) / kScanTile)
     need += t + 1;
   cudaError_t e = ctx->s_scan.ensure(need * sizeof(uint32_t));
   if (e != cudaSuccess) return cuda_status(e, "scan scratch");
-  return scan_levels(ctx->stream, in, out, n, ctx->s_scan.as<uint32_t>(), ctx->launches);
+  return scan_levels(ctx->stream, in, out, n, ctx->s_scan.as<uint32_t>(), ctx->launches, skip);
 }
 
 srt_status scan_exclusive(srt_ctx *ctx, const uint32_t *in, uint32_t *out, size_t n) {
@@ -588,7 +594,8 @@ template <bool SEGDIG, int BITS>
 __global__ void __launch_bounds__(kRsThreads)
 rs_hist_kernel(const uint32_t *__restrict__ keys, const uint32_t *__restrict__ vals,
                size_t n, int shift, uint32_t *__restrict__ hist, uint32_t ntiles,
-               const uint32_t *__restrict__ seg, int nseg) {
+               const uint32_t *__restrict__ seg, int nseg, const uint32_t *__restrict__ skip) {
+  if (skip && *skip) return;
   constexpr int kBins = 1 << BITS;
   __shared__ uint32_t wh[kRsWarps][kBins];
   for (int i = threadIdx.x; i < kRsWarps * kBins; i += kRsThreads)
@@ -624,7 +631,8 @@ __global__ void __launch_bounds__(kRsThreads)
 rs_scatter_kernel(const uint32_t *__restrict__ kin, const uint32_t *__restrict__ vin,
                   uint32_t *__restrict__ kout, uint32_t *__restrict__ vout, size_t n,
                   int shift, const uint32_t *__restrict__ offs, uint32_t ntiles,
-                  const uint32_t *__restrict__ seg, int nseg) {
+                  const uint32_t *__restrict__ seg, int nseg, const uint32_t *__restrict__ skip) {
+  if (skip && *skip) return;
   constexpr int kBins = 1 << BITS;
   __shared__ uint32_t wc[kRsWarps][kBins];
   for (int i = threadIdx.x; i < kRsWarps * kBins; i += kRsThreads)
@@ -701,19 +709,19 @@ rs_scatter_kernel(const uint32_t *__restrict__ kin, const uint32_t *__restrict__
 template <bool SEGDIG, int BITS>
 static srt_status sort_pass(srt_ctx *ctx, const uint32_t *k0, const uint32_t *v0,
                             uint32_t *k1, uint32_t *v1, size_t n, int shift,
-                            const uint32_t *seg, int nseg) {
+                            const uint32_t *seg, int nseg, const uint32_t *skip = nullptr) {
   cudaStream_t st = ctx->stream;
   const uint32_t ntiles = (uint32_t)((n + kRsTile - 1) / kRsTile);
   uint32_t *hist = ctx->s_hist.as<uint32_t>();
   rs_hist_kernel<SEGDIG, BITS><<<ntiles, kRsThreads, 0, st>>>(k0, v0, n, shift, hist, ntiles,
-                                                              seg, nseg);
+                                                              seg, nseg, skip);
   ctx->launches++;
   srt_status s = cuda_status(cudaGetLastError(), "rs_hist");
   if (s != SRT_OK) return s;
-  s = exclusive_scan(ctx, hist, hist, (size_t)(1u << BITS) * ntiles);
+  s = exclusive_scan(ctx, hist, hist, (size_t)(1u << BITS) * ntiles, skip);
   if (s != SRT_OK) return s;
   rs_scatter_kernel<SEGDIG, BITS><<<ntiles, kRsThreads, 0, st>>>(k0, v0, k1, v1, n, shift,
-                                                                 hist, ntiles, seg, nseg);
+                                                                 hist, ntiles, seg, nseg, skip);
   ctx->launches++;
   return cuda_status(cudaGetLastError(), "rs_scatter");
 }
@@ -735,7 +743,8 @@ static srt_status sort_scratch(srt_ctx *ctx, size_t n) {
 // result by the segment of each value (the segment offsets `seg` are global
 // indices), i.e. the order is (segment, key, value).
 srt_status sort_pairs_seg(srt_ctx *ctx, uint32_t *keys, uint32_t *vals, size_t n,
-                          bool identity_vals, const uint32_t *seg, int nseg, int key_bits) {
+                          bool identity_vals, const uint32_t *seg, int nseg, int key_bits,
+                          const uint32_t *skip = nullptr) {
   if (n == 0) return SRT_OK;
   srt_status s = sort_scratch(ctx, n);
   if (s != SRT_OK) return s;
@@ -745,8 +754,8 @@ srt_status sort_pairs_seg(srt_ctx *ctx, uint32_t *keys, uint32_t *vals, size_t n
   const int passes = narrow ? (key_bits < 1 ? 1 : (key_bits + 9) / 10) : 4;
   for (int pass = 0; pass < passes; pass++) {
     const uint32_t *vin = (pass == 0 && identity_vals) ? nullptr : v0;
-    s = narrow ? sort_pass<false, 10>(ctx, k0, vin, k1, v1, n, pass * 10, nullptr, 0)
-               : sort_pass<false, 8>(ctx, k0, vin, k1, v1, n, pass * 8, nullptr, 0);
+    s = narrow ? sort_pass<false, 10>(ctx, k0, vin, k1, v1, n, pass * 10, nullptr, 0, skip)
+               : sort_pass<false, 8>(ctx, k0, vin, k1, v1, n, pass * 8, nullptr, 0, skip);
     if (s != SRT_OK) return s;
     std::swap(k0, k1);
     std::swap(v0, v1);
@@ -767,8 +776,8 @@ srt_status sort_pairs_seg(srt_ctx *ctx, uint32_t *keys, uint32_t *vals, size_t n
 }
 
 srt_status sort_pairs(srt_ctx *ctx, uint32_t *keys, uint32_t *vals, size_t n,
-                      bool identity_vals, int key_bits) {
-  return sort_pairs_seg(ctx, keys, vals, n, identity_vals, nullptr, 1, key_bits);
+                      bool identity_vals, int key_bits, const uint32_t *skip) {
+  return sort_pairs_seg(ctx, keys, vals, n, identity_vals, nullptr, 1, key_bits, skip);
 }
 
 namespace {

@@ -187,7 +187,7 @@ struct srt_ctx {
       s_kparent, s_lparent, s_counter, s_ibox, s_flag, s_slot, s_partial,
       s_stage_in, s_stage_out, s_stage_aux, s_stage_sub, s_stage_scal, s_stage_norm,
       s_defer, s_spawn, s_rkey, s_rorder, s_isect_sub, s_stage_isect, s_keys3, s_vals3,
-      s_status, s_lscan, s_rays_in, s_kidx, s_kprefix;
+      s_status, s_lscan, s_rays_in, s_kidx, s_kprefix, s_raster;
   uint32_t os_epoch = 0;  // look-back epoch of the last sort pass (srt_sort.cu)
   // recorded after a build's host inputs were copied; the next staged ray
   // array waits for it (inputs_pending)
@@ -351,8 +351,15 @@ void build_top_tree(const double *bmin, const double *bmax, size_t n,
 // line or solid element's tree is deeper than 62 levels.
 srt_status launch_scene_trace(srt_ctx *ctx, const TopNode *top, SceneWork W, uint32_t kinds,
                               bool deep_lines, const SceneStreams &ss);
-// Coherent traversal order of n rays (srt_raysort.cu): *order is a device
-// array in context scratch, valid until the context's next sort.
+// Rays of a camera, which come in rows, in square tiles of them, any other
+// rays in array order (srt_raysort.cu): *order is a device array in context
+// scratch, valid until the context's next order.  With roff (ray offsets of
+// nseg segments, on the device) each segment is a set of its own.
+srt_status raster_order(srt_ctx *ctx, const srt_ray *rays, size_t n, const uint32_t **order);
+srt_status raster_order(srt_ctx *ctx, const srt_ray *rays, size_t n, const uint32_t *roff,
+                        int nseg, uint32_t *order);
+// Coherent traversal order of n rays (srt_raysort.cu), by tiles of rows or a
+// sort: *order as above.
 srt_status ray_order(srt_ctx *ctx, const srt_ray *rays, size_t n, const uint32_t **order);
 // The same for the rays of a batch (ray offsets roff over nseg scenes, on
 // the device), kept grouped by scene, ordered within a scene by the top
@@ -371,9 +378,11 @@ bool solid_scene_view(const srt_solid_accel *a, srt_ctx **ctx, SceneElem &e, boo
 // Exclusive prefix sum of n uint32 on the context's stream (out may alias in).
 srt_status scan_exclusive(srt_ctx *ctx, const uint32_t *in, uint32_t *out, size_t n);
 // Stable sort of (key, value) pairs by key; key_bits: how many low bits of
-// the keys can be non-zero (30 for Morton codes).
+// the keys can be non-zero (30 for Morton codes); skip: a device word that,
+// when set, makes the kernels return (the arrays are then unspecified).
 srt_status sort_pairs(srt_ctx *ctx, uint32_t *d_keys, uint32_t *d_vals,
-                      size_t n, bool identity_vals, int key_bits = 32);
+                      size_t n, bool identity_vals, int key_bits = 32,
+                      const uint32_t *skip = nullptr);
 // The same order for 30-bit keys (Morton codes) with one kernel per 10-bit
 // pass (srt_sort.cu); n < 2^30.
 srt_status sort_codes30(srt_ctx *ctx, uint32_t *d_keys, uint32_t *d_vals, size_t n,
