@@ -1275,7 +1275,10 @@ __global__ void widen_kernel(const Node2 *__restrict__ nodes,
                              const uint32_t *__restrict__ nbranches, uint32_t cap,
                              WideRec *__restrict__ wide, uint32_t *__restrict__ irregular) {
   const uint32_t nb = *nbranches;
-  if (nb > cap) return;  // the two-child nodes are walked instead
+  if (nb > cap) {  // the two-child nodes are walked instead, their boxes unseen
+    if (blockIdx.x == 0 && threadIdx.x == 0) *irregular = 1u;
+    return;
+  }
   for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < 4 * nb;
        t += gridDim.x * blockDim.x) {
     const Box2 p = node2_child(nodes[t >> 2], (t >> 1) & 1u);
@@ -1795,7 +1798,7 @@ __global__ void seg_emit_node2_kernel(const uint32_t *__restrict__ codes,
                                       const uint32_t *__restrict__ slot,
                                       const Box *__restrict__ ibox,
                                       const float4 *__restrict__ prims,
-                                      const SceneInfo *__restrict__ scenes,
+                                      SceneInfo *__restrict__ scenes,
                                       const uint32_t *__restrict__ foff,
                                       const uint32_t *__restrict__ ioff, int nseg, uint32_t M,
                                       Node2 *__restrict__ nodes, uint32_t *__restrict__ err) {
@@ -1827,6 +1830,9 @@ __global__ void seg_emit_node2_kernel(const uint32_t *__restrict__ codes,
         }
       }
       if (cnt[side] > kCountMask) atomicOr(err, kErrTree);
+#pragma unroll
+      for (int k = 0; k < 3; k++)
+        if (!(bx[side].lo[k] <= bx[side].hi[k])) scenes[sg].irregular = 1u;
     }
     const uint32_t axis = (uint32_t)split_axis(codes[fb + (g - ib)]);
     Node2 nd;

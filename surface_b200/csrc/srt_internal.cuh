@@ -58,8 +58,8 @@ struct __align__(16) Node2 {
 struct __align__(32) WideRec {
   float4 a, b;
 };
-// SceneInfo.irregular: some box of the wide nodes is not ordered (lo <= hi,
-// false for NaN) or not inside its parent's.
+// SceneInfo.irregular: some box of the tree is not ordered (lo <= hi, false
+// for NaN) or, of the wide nodes, not inside its parent's.
 
 // Own-box node (tetrahedra): 32 bytes, the reference's TetraNode.
 //   a = (lo.x, lo.y, lo.z, meta)  meta: leaf -> kLeafBit | count, branch -> axis

@@ -748,6 +748,64 @@ struct SharedStack {
   __shared__ float NAME##_t[kShDepth][NT];                 \
   SharedStack<NT> NAME(NAME##_e, NAME##_t)
 
+// Two floats as one 64-bit operand of the packed instructions: each half is
+// added and multiplied with its own IEEE rounding.
+__device__ __forceinline__ float2 add2(float2 a, float2 b) {
+  unsigned long long r;
+  asm("add.rn.f32x2 %0, %1, %2;"
+      : "=l"(r)
+      : "l"(*reinterpret_cast<unsigned long long *>(&a)),
+        "l"(*reinterpret_cast<unsigned long long *>(&b)));
+  return *reinterpret_cast<float2 *>(&r);
+}
+__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
+  unsigned long long r;
+  asm("mul.rn.f32x2 %0, %1, %2;"
+      : "=l"(r)
+      : "l"(*reinterpret_cast<unsigned long long *>(&a)),
+        "l"(*reinterpret_cast<unsigned long long *>(&b)));
+  return *reinterpret_cast<float2 *>(&r);
+}
+
+// A component the slab test's products can turn into NaN.
+__device__ __forceinline__ bool odd_ray(const RayF &r) {
+  bool odd = false;
+#pragma unroll
+  for (int k = 0; k < 3; k++)
+    odd = odd || !(fabsf(r.o[k]) <= FLT_MAX) || !(fabsf(r.inv[k]) <= FLT_MAX) || r.inv[k] == 0.0f;
+  return odd;
+}
+
+// The slab test of boxes that are ordered (lo <= hi) by a ray that is not
+// odd: no product is NaN and the smaller of a slab's two distances is the
+// entry whatever the direction's sign, so minima and maxima give what the
+// reference's selections give, and its subtractions and products go in
+// pairs -- 24 instructions a box instead of 36.  With the sphere prefilter
+// of pass1_node2: 8 M spheres, 1024^2 rays 727 M -> 470 M warp instructions;
+// 16.8 M spheres, 2048^2 and their bounces 6.35 -> 5.63 ms, 64 triangle
+// scenes 6.06 -> 5.63 ms.  (16-byte stack entries were slower: 5.91 and
+// 5.80 ms; 8 blocks per SM by launch bounds 5.90 and 5.62.)  The six coordinates of a box
+// as two-child nodes store them: (lo.x, lo.y), (lo.z, hi.x), (hi.y, hi.z).
+struct SlabRay {
+  float2 o01, o20, o12, i01, i20, i12;  // -origin and reciprocal, paired alike
+  __device__ __forceinline__ explicit SlabRay(const RayF &r) {
+    o01 = make_float2(-r.o[0], -r.o[1]);
+    o20 = make_float2(-r.o[2], -r.o[0]);
+    o12 = make_float2(-r.o[1], -r.o[2]);
+    i01 = make_float2(r.inv[0], r.inv[1]);
+    i20 = make_float2(r.inv[2], r.inv[0]);
+    i12 = make_float2(r.inv[1], r.inv[2]);
+  }
+  __device__ __forceinline__ bool hit(float2 a, float2 b, float2 c, float bnd, float &tmin) const {
+    const float2 p = mul2(add2(a, o01), i01);  // x0, y0
+    const float2 q = mul2(add2(b, o20), i20);  // z0, x1
+    const float2 s = mul2(add2(c, o12), i12);  // y1, z1
+    tmin = fmaxf(fmaxf(fminf(p.x, q.y), fminf(p.y, s.x)), fminf(q.x, s.y));
+    const float tmax = fminf(fminf(fmaxf(p.x, q.y), fmaxf(p.y, s.x)), fmaxf(q.x, s.y));
+    return tmax > 0.0f && tmin <= fminf(tmax, bnd);
+  }
+};
+
 // Pass 1 of the default walk for the two-child kinds: front to back from
 // `root`; returns m (smallest hit distance), how many primitives hit at m,
 // the one found first (in b), and whether one of those at m was reported
@@ -757,9 +815,12 @@ __device__ __forceinline__ void pass1_node2(const Node2 *__restrict__ nodes,
                                             const float4 *__restrict__ prims,
                                             const uint32_t *__restrict__ sidx,
                                             const Ctx2 &c, uint32_t root, Best &b, Work &w,
-                                            uint32_t max_iter, float &m_out,
+                                            uint32_t max_iter, bool irregular, float &m_out,
                                             uint32_t &at_m_out, bool &viol_out,
                                             Stk &&stk = Stk()) {
+  const bool odd = irregular || odd_ray(c.r);
+  const SlabRay slab(c.r);
+  const float ray_a = dot3(c.r.d, c.r.d);
   float m = FLT_MAX, m2 = FLT_MAX;  // smallest and second smallest distance
   float e_best = 0.0f;              // leaf box entry of the candidate at m
   uint32_t at_m = 0;
@@ -782,8 +843,14 @@ __device__ __forceinline__ void pass1_node2(const Node2 *__restrict__ nodes,
       const float4 a = __ldg(np), bb = __ldg(np + 1), cc = __ldg(np + 2);
       const uint4 d = __ldg(reinterpret_cast<const uint4 *>(np + 3));
       float t0, t1;
-      const bool h0 = ray_aabb_t<true>(bnd, a.x, a.y, a.z, a.w, bb.x, bb.y, c.r, t0);
-      const bool h1 = ray_aabb_t<true>(bnd, bb.z, bb.w, cc.x, cc.y, cc.z, cc.w, c.r, t1);
+      bool h0 = slab.hit(make_float2(a.x, a.y), make_float2(a.z, a.w), make_float2(bb.x, bb.y), bnd,
+                         t0);
+      bool h1 = slab.hit(make_float2(bb.z, bb.w), make_float2(cc.x, cc.y),
+                         make_float2(cc.z, cc.w), bnd, t1);
+      if (odd) {
+        h0 = ray_aabb_t<true>(bnd, a.x, a.y, a.z, a.w, bb.x, bb.y, c.r, t0);
+        h1 = ray_aabb_t<true>(bnd, bb.z, bb.w, cc.x, cc.y, cc.z, cc.w, c.r, t1);
+      }
       const uint2 e0 = make_uint2(d.x, d.z & kCountMask),
                   e1 = make_uint2(d.y, d.w & kCountMask);
       if (sp + 2 >= std::remove_reference_t<Stk>::kDepth) { w.fail = true; sp = -1; break; }
@@ -800,26 +867,49 @@ __device__ __forceinline__ void pass1_node2(const Node2 *__restrict__ nodes,
     if (leaf.y == 0) break;
     w.leaf++;
     w.prim += leaf.y;
-    // primitive j + 1 is loaded while j is tested
-    Prim2<KIND> nx;
-    nx.load(prims, sidx, leaf.x);
-    for (uint32_t j = leaf.x; j < leaf.x + leaf.y; j++) {
-      const Prim2<KIND> P = nx;
-      if (j + 1 < leaf.x + leaf.y) nx.load(prims, sidx, j + 1);
-      float t, u, v;
-      if (!P.test(c, FLT_MAX, t, u, v)) continue;
+    auto take = [&](float t, float u, float v, uint32_t f, uint32_t j) {
       if (t < m) {
         m2 = m;
         m = t;
         at_m = 1;
         viol = below_entry(t, lt);
         e_best = lt;
-        b.t = t; b.u = u; b.v = v; b.prim = P.f; b.j = j;
+        b.t = t; b.u = u; b.v = v; b.prim = f; b.j = j;
       } else {
         if (t < m2) m2 = t;
         if (t == m) {
           at_m++;
           viol = viol || below_entry(t, lt);
+        }
+      }
+    };
+    const uint32_t end = leaf.x + leaf.y;
+    if (KIND == SRT_TRIANGLES) {
+      // primitive j + 1 is loaded while j is tested
+      Prim2<KIND> nx;
+      nx.load(prims, sidx, leaf.x);
+      for (uint32_t j = leaf.x; j < end; j++) {
+        const Prim2<KIND> P = nx;
+        if (j + 1 < end) nx.load(prims, sidx, j + 1);
+        float t, u, v;
+        if (P.test(c, FLT_MAX, t, u, v)) take(t, u, v, P.f, j);
+      }
+    } else {
+      // most spheres of a leaf are missed: those whose discriminant is surely
+      // negative are dropped first, so that the square root and divisions
+      // run for one or two of a leaf instead of all
+      for (uint32_t j0 = leaf.x; j0 < end; j0 += 32) {
+        const uint32_t cnt = min(end - j0, 32u);
+        unsigned maybe = 0;
+        for (uint32_t q = 0; q < cnt; q++)
+          if (sphere_maybe(__ldg(&prims[j0 + q]), c.r, ray_a)) maybe |= 1u << q;
+        while (maybe) {
+          const uint32_t j = j0 + (uint32_t)(__ffs(maybe) - 1);
+          maybe &= maybe - 1;
+          Prim2<KIND> P;
+          P.load(prims, sidx, j);
+          float t, u, v;
+          if (P.test(c, FLT_MAX, t, u, v)) take(t, u, v, P.f, j);
         }
       }
     }
@@ -884,34 +974,6 @@ struct Group {
     return fminf(v, other(v, 2));
   }
 };
-
-// Two floats as one 64-bit operand of the packed instructions: each half is
-// added and multiplied with its own IEEE rounding.
-__device__ __forceinline__ float2 add2(float2 a, float2 b) {
-  unsigned long long r;
-  asm("add.rn.f32x2 %0, %1, %2;"
-      : "=l"(r)
-      : "l"(*reinterpret_cast<unsigned long long *>(&a)),
-        "l"(*reinterpret_cast<unsigned long long *>(&b)));
-  return *reinterpret_cast<float2 *>(&r);
-}
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
-  unsigned long long r;
-  asm("mul.rn.f32x2 %0, %1, %2;"
-      : "=l"(r)
-      : "l"(*reinterpret_cast<unsigned long long *>(&a)),
-        "l"(*reinterpret_cast<unsigned long long *>(&b)));
-  return *reinterpret_cast<float2 *>(&r);
-}
-
-// A component the slab test's products can turn into NaN.
-__device__ __forceinline__ bool odd_ray(const RayF &r) {
-  bool odd = false;
-#pragma unroll
-  for (int k = 0; k < 3; k++)
-    odd = odd || !(fabsf(r.o[k]) <= FLT_MAX) || !(fabsf(r.inv[k]) <= FLT_MAX) || r.inv[k] == 0.0f;
-  return odd;
-}
 
 // A lane's candidates: the smallest distance m with its barycentrics and
 // sorted primitive, its leaf box's entry, the second smallest distance, and
@@ -1241,6 +1303,7 @@ trace_node2_kernel(const Node2 *__restrict__ nodes, const float4 *__restrict__ p
                    uint32_t *__restrict__ err, const uint32_t *__restrict__ order,
                    uint32_t *__restrict__ next = nullptr, uint32_t wide_cap = 0) {
   if (wide_cap && scene->nbranches <= wide_cap) return;  // trace_wide_kernel traced the rays
+  const bool irregular = scene->irregular != 0;
   for_each_ray(n, next, [&](size_t k) {
     const size_t i = order ? (size_t)__ldg(&order[k]) : k;  // ray of this thread
     const Ctx2 c = make_ctx2<KIND>(rays, i, scene, prev_normals);
@@ -1252,7 +1315,7 @@ trace_node2_kernel(const Node2 *__restrict__ nodes, const float4 *__restrict__ p
       float m;
       uint32_t at_m;
       bool viol;
-      pass1_node2<KIND>(nodes, prims, sidx, c, 0u, b, w, max_iter, m, at_m, viol);
+      pass1_node2<KIND>(nodes, prims, sidx, c, 0u, b, w, max_iter, irregular, m, at_m, viol);
       if (!w.fail && (viol || at_m > 1)) {
         const uint32_t q = atomicAdd(dcount, 1u);
         dlist[q] = Deferred{(uint32_t)i, viol ? 1u : 0u, (double)m};
@@ -1958,7 +2021,7 @@ trace_batch_kernel(const Node2 *__restrict__ nodes, const float4 *__restrict__ p
       uint32_t at_m;
       bool viol;
       pass1_node2<SRT_TRIANGLES>(nodes, prims, nullptr, c, __ldg(&roots[sg]), b, w, max_iter,
-                                 m, at_m, viol, LocalStackN<DEPTH>());
+                                 scenes[sg].irregular != 0, m, at_m, viol, LocalStackN<DEPTH>());
       if (!w.fail && (viol || at_m > 1)) {
         const uint32_t q = atomicAdd(dcount, 1u);
         dlist[q] = Deferred{i, viol ? 1u : 0u, (double)m};
@@ -2415,7 +2478,7 @@ __device__ __forceinline__ bool elem_pass1(const SceneElem &e, const typename Ki
     uint32_t at_m;
     bool viol;
     pass1_node2<KIND>(static_cast<const Node2 *>(e.nodes), e.prims, e.sidx, c, 0u, b, w,
-                      max_iter, mf, at_m, viol);
+                      max_iter, e.scene->irregular != 0, mf, at_m, viol);
     m = mf;
     full = viol;
     return w.fail || !(viol || at_m > 1);
