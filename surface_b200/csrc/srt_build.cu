@@ -736,6 +736,9 @@ static srt_status sort_scratch(srt_ctx *ctx, size_t n) {
   return SRT_OK;
 }
 
+// Keys of 21 to 30 bits: from here on sort_codes30_large.
+constexpr size_t kLargeSort = (size_t)1 << 17;
+
 // Stable LSD sort of (keys, vals) by key; result lands back in keys/vals.
 // identity_vals: vals are 0..n-1 on entry (not read).  key_bits <= 30: one
 // 10-bit pass per 10 bits (three for Morton codes), otherwise four 8-bit
@@ -746,6 +749,10 @@ srt_status sort_pairs_seg(srt_ctx *ctx, uint32_t *keys, uint32_t *vals, size_t n
                           bool identity_vals, const uint32_t *seg, int nseg, int key_bits,
                           const uint32_t *skip = nullptr) {
   if (n == 0) return SRT_OK;
+  // (larger batches of scenes than a digit tells apart, and other keys, take
+  // the passes below)
+  if (key_bits > 20 && key_bits <= 30 && n > kLargeSort && n < (1u << 30) && nseg <= 256)
+    return sort_codes30_large(ctx, keys, vals, n, identity_vals, seg, nseg, skip);
   srt_status s = sort_scratch(ctx, n);
   if (s != SRT_OK) return s;
   uint32_t *k0 = keys, *v0 = vals, *k1 = ctx->s_keys2.as<uint32_t>(),

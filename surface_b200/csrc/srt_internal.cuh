@@ -187,7 +187,7 @@ struct srt_ctx {
       s_kparent, s_lparent, s_counter, s_ibox, s_flag, s_slot, s_partial,
       s_stage_in, s_stage_out, s_stage_aux, s_stage_sub, s_stage_scal, s_stage_norm,
       s_defer, s_spawn, s_rkey, s_rorder, s_isect_sub, s_stage_isect, s_keys3, s_vals3,
-      s_status, s_lscan, s_rays_in, s_kidx, s_kprefix, s_raster, s_brick;
+      s_status, s_lscan, s_rays_in, s_kidx, s_kprefix, s_raster, s_brick, s_status_lg;
   uint32_t os_epoch = 0;  // look-back epoch of the last sort pass (srt_sort.cu)
   // recorded after a build's host inputs were copied; the next staged ray
   // array waits for it (inputs_pending)
@@ -387,7 +387,13 @@ srt_status sort_pairs(srt_ctx *ctx, uint32_t *d_keys, uint32_t *d_vals,
 // pass (srt_sort.cu); n < 2^30.
 srt_status sort_codes30(srt_ctx *ctx, uint32_t *d_keys, uint32_t *d_vals, size_t n,
                         bool identity_vals, bool hist_ready = false);
-// Its scratch for n keys: the digit histograms (3 x 1024 words, to be filled
+// The same order for large arrays (8-bit passes over long tiles), then with
+// nseg > 1 (at most 256) a pass that groups it by the segment of each value,
+// seg the segments' offsets on the device; skip as for sort_pairs.
+srt_status sort_codes30_large(srt_ctx *ctx, uint32_t *d_keys, uint32_t *d_vals, size_t n,
+                              bool identity_vals, const uint32_t *seg = nullptr, int nseg = 1,
+                              const uint32_t *skip = nullptr);
+// Scratch of sort_codes30 for n keys: the digit histograms (3 x 1024 words, to be filled
 // before a hist_ready sort) and the three passes' tile counters (zeroed).
 srt_status sort_codes30_scratch(srt_ctx *ctx, size_t n, uint32_t **hist,
                                 unsigned long long **tickets);
