@@ -184,7 +184,7 @@ struct srt_ctx {
   uint64_t launches = 0;  // kernels launched by this context
   // scratch shared by the builds of this context (stream ordered)
   srt::DevBuf s_keys2, s_vals2, s_hist, s_scan, s_kchild, s_kflags, s_krange,
-      s_kparent, s_lparent, s_counter, s_ibox, s_flag, s_slot, s_partial,
+      s_kparent, s_counter, s_ibox, s_flag, s_slot, s_partial,
       s_stage_in, s_stage_out, s_stage_aux, s_stage_sub, s_stage_scal, s_stage_norm,
       s_defer, s_spawn, s_rkey, s_rorder, s_isect_sub, s_stage_isect, s_keys3, s_vals3,
       s_status, s_lscan, s_rays_in, s_kidx, s_kprefix, s_raster, s_brick, s_status_lg;
