@@ -281,8 +281,9 @@ constexpr int32_t kTetAuxDouble = 512;
 // One element of a scene: a built accel and its transforms, 4x4 doubles in
 // the reference's Matrixd layout (m[row][col], p' = p m + m[3]).  Line and
 // solid elements keep their device nodes in nodes and records in prims;
-// aux: the line accel's cap flag, the solid accel's vertices per solid (|
-// kSolidAuxDouble for double-precision positions).
+// aux: the line accel's flags (1: caps, 2: every box is ordered), the solid
+// accel's vertices per solid (| kSolidAuxDouble for double-precision
+// positions).
 struct SceneElem {
   int32_t kind;
   uint32_t nprims;
@@ -370,7 +371,7 @@ srt_status batch_ray_order(srt_ctx *ctx, const srt_ray *rays, size_t n, const ui
 uint64_t line_accel_bytes(const srt_line_accel *a);
 uint64_t solid_accel_bytes(const srt_solid_accel *a);
 // A built line or solid accel as a scene element: its context, device
-// nodes and records, element count, aux (cap flag / vertices per solid)
+// nodes and records, element count, aux (see SceneElem)
 // and tree depth (lines) or whether the tree is deeper than 62 levels
 // (solids).  False when the accel is not built.
 bool line_scene_view(const srt_line_accel *a, srt_ctx **ctx, SceneElem &e, int &depth);

@@ -13,12 +13,11 @@
 // cap plane normal and offsets), computed with the reference's float
 // operations.
 //
-// Trace (LineAccel::Traverse, :704-774): one thread per ray (in a Morton
-// order of the rays for large batches), the stack of
-// the reference (a popped branch tests its own box against the closest hit
-// so far, then pushes far and near children by the sign of the ray's
-// direction on the branch's axis), every line of a popped leaf tested in
-// order by CylinderIsect (:488-577).  Compiled without FMA contraction; the
+// Trace (LineAccel::Traverse, :704-774): one thread per ray (in tiles of the
+// rays' rows or a Morton order for large batches), in the reference's order
+// (a branch's box against the closest hit so far, then its near and its far
+// child by the sign of the ray's direction on the branch's axis), every line
+// of an entered leaf tested in order by CylinderIsect (:488-577).  Compiled without FMA contraction; the
 // reference's unqualified sqrt and fabs are the double C functions, so the
 // quadratic's first root is formed in double, and every other sqrt and
 // reciprocal rounds as the float operation does.
@@ -56,6 +55,7 @@ struct srt_line_accel {
   std::vector<LineNodeH> nodes;
   std::vector<uint32_t> idx;
   srt::DevBuf dnodes, drecs;
+  bool ordered = false;          // every box has bmin <= bmax
   // build scratch, kept between builds (grown by doubling)
   srt::DevBuf s_lbox, s_mid, s_node_of, s_pairs, s_bsum, s_level, s_nchild, s_cbase, s_bfs,
       s_sizes, s_pre, s_cnt;
@@ -505,7 +505,8 @@ __global__ void lvl_size_kernel(const LBNode *__restrict__ nodes, uint32_t off, 
 
 __global__ void lvl_emit_kernel(const LBNode *__restrict__ nodes, uint32_t off, uint32_t m,
                                 const uint32_t *__restrict__ size, uint32_t *__restrict__ pre,
-                                LineNodeH *__restrict__ ref, LNode *__restrict__ dev) {
+                                LineNodeH *__restrict__ ref, LNode *__restrict__ dev,
+                                uint32_t *__restrict__ bad) {
   for (uint32_t v = blockIdx.x * blockDim.x + threadIdx.x; v < m; v += gridDim.x * blockDim.x) {
     const uint32_t g = off + v;
     const LBNode nd = nodes[g];
@@ -513,6 +514,7 @@ __global__ void lvl_emit_kernel(const LBNode *__restrict__ nodes, uint32_t off, 
     LineNodeH h;
     LNode d;
     for (int k = 0; k < 3; k++) {
+      if (!(nd.bmin[k] <= nd.bmax[k])) *bad = 1u;
       h.bmin[k] = d.bmin[k] = nd.bmin[k];
       h.bmax[k] = d.bmax[k] = nd.bmax[k];
     }
@@ -573,10 +575,10 @@ __global__ void line_rec_kernel(const float *__restrict__ pos, const float *__re
 // ray order[k].  STATS: count popped branches, popped leaves and line tests
 // into stats[0..2].
 template <int STACK, bool STATS>
-__global__ void __launch_bounds__(128)
+__global__ void __launch_bounds__(128, STACK <= 64 ? 8 : 1)
 line_trace_kernel(const LNode *__restrict__ nodes, const LineRec *__restrict__ recs, bool cap,
-                  const srt_ray *__restrict__ rays, const uint32_t *__restrict__ order,
-                  size_t n, srt_hit *__restrict__ hits, float *__restrict__ normals,
+                  bool ordered, const srt_ray *__restrict__ rays,
+                  const uint32_t *__restrict__ order, size_t n, srt_hit *__restrict__ hits, float *__restrict__ normals,
                   unsigned long long *__restrict__ stats) {
   unsigned long long nb = 0, nl = 0, nt = 0;
   for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n;
@@ -586,7 +588,7 @@ line_trace_kernel(const LNode *__restrict__ nodes, const LineRec *__restrict__ r
     const float4 r0 = __ldg(rq), r1 = __ldg(rq + 1);
     const float ro[3] = {r0.x, r0.y, r0.z}, rdir[3] = {r1.x, r1.y, r1.z};
     const RayL R = make_ray(ro, rdir);
-    const LineHit H = line_walk<STACK, STATS>(nodes, recs, cap, R, nb, nl, nt);
+    const LineHit H = line_walk<STACK, STATS>(nodes, recs, cap, ordered, R, nb, nl, nt);
     const float it = H.t, iu = H.u, iv = H.v;
     const bool icap = H.cap;
     const int best = H.rec;
@@ -663,7 +665,7 @@ bool line_scene_view(const srt_line_accel *a, srt_ctx **ctx, SceneElem &e, int &
   *ctx = a->ctx;
   e.kind = kSceneLines;
   e.nprims = (uint32_t)a->nlines;
-  e.aux = a->cap;
+  e.aux = a->cap | (a->ordered ? 2 : 0);
   e.nodes = a->dnodes.p;
   e.prims = a->drecs.as<float4>();
   e.sidx = nullptr;
@@ -759,7 +761,7 @@ SRT_API srt_status srt_line_build(srt_line_accel *a, const float *positions, siz
       (e = grow(bsum, ((size_t)tiles + 1) * 4)) != cudaSuccess ||
       (e = grow(cnt, 16)) != cudaSuccess)
     return cuda_status(e, "line build scratch");
-  uint32_t *d_err = cnt.as<uint32_t>(), *d_pairs = d_err + 1, *d_next = d_err + 2;
+  uint32_t *d_err = cnt.as<uint32_t>(), *d_pairs = d_err + 1, *d_next = d_err + 2, *d_bad = d_err + 3;
   cudaMemsetAsync(d_err, 0, 16, st);
   const unsigned egrid = (unsigned)std::min<size_t>((n + 255) / 256, (size_t)ctx->num_sms * 16);
   line_prep_kernel<<<egrid, 256, 0, st>>>(
@@ -862,7 +864,7 @@ SRT_API srt_status srt_line_build(srt_line_accel *a, const float *positions, siz
   for (const auto &[lo, cntl] : levels)
     lvl_emit_kernel<<<(unsigned)std::min<size_t>(((size_t)cntl + 255) / 256, 65535), 256, 0, st>>>(
         bfs.as<LBNode>(), lo, cntl, sizes.as<uint32_t>(), pre.as<uint32_t>(),
-        a->dref.as<LineNodeH>(), a->dnodes.as<LNode>());
+        a->dref.as<LineNodeH>(), a->dnodes.as<LNode>(), d_bad);
   ctx->launches += 2 * levels.size();
   const unsigned grid = (unsigned)std::min<size_t>((n + 255) / 256, 4096);
   line_rec_kernel<<<grid, 256, 0, st>>>(
@@ -871,11 +873,14 @@ SRT_API srt_status srt_line_build(srt_line_accel *a, const float *positions, siz
   ctx->launches++;
   if ((e = cudaGetLastError()) != cudaSuccess) return cuda_status(e, "line records");
   cudaMemcpyAsync(&a->root, a->dref.p, sizeof(LineNodeH), cudaMemcpyDeviceToHost, st);
+  uint32_t bad = 0;
+  cudaMemcpyAsync(&bad, d_bad, 4, cudaMemcpyDeviceToHost, st);
   // the staged inputs are freed on return: finish with them first
   if ((e = cudaStreamSynchronize(st)) != cudaSuccess) return cuda_status(e, "line build");
   a->nlines = n;
   a->nnodes = total;
   a->depth = (int)levels.size() - 1;
+  a->ordered = bad == 0;
   a->cap = cap != 0;
   a->built = true;
   return SRT_OK;
@@ -927,16 +932,16 @@ SRT_API srt_status srt_line_trace(srt_line_accel *a, const srt_ray *rays, size_t
   if (n >= 32768 && (s = ray_order(ctx, rr, n, &ord)) != SRT_OK) return s;
   const bool shallow = a->depth + 2 <= 64;
   if (shallow && !st)
-    line_trace_kernel<64, false><<<grid, 128, 0, ctx->stream>>>(nd, rc, a->cap, rr, ord, n, dh,
+    line_trace_kernel<64, false><<<grid, 128, 0, ctx->stream>>>(nd, rc, a->cap, a->ordered, rr, ord, n, dh,
                                                                  dn, st);
   else if (shallow)
-    line_trace_kernel<64, true><<<grid, 128, 0, ctx->stream>>>(nd, rc, a->cap, rr, ord, n, dh,
+    line_trace_kernel<64, true><<<grid, 128, 0, ctx->stream>>>(nd, rc, a->cap, a->ordered, rr, ord, n, dh,
                                                                 dn, st);
   else if (!st)
-    line_trace_kernel<520, false><<<grid, 128, 0, ctx->stream>>>(nd, rc, a->cap, rr, ord, n, dh,
+    line_trace_kernel<520, false><<<grid, 128, 0, ctx->stream>>>(nd, rc, a->cap, a->ordered, rr, ord, n, dh,
                                                                   dn, st);
   else
-    line_trace_kernel<520, true><<<grid, 128, 0, ctx->stream>>>(nd, rc, a->cap, rr, ord, n, dh,
+    line_trace_kernel<520, true><<<grid, 128, 0, ctx->stream>>>(nd, rc, a->cap, a->ordered, rr, ord, n, dh,
                                                                  dn, st);
   ctx->launches++;
   if ((e = cudaGetLastError()) != cudaSuccess) return cuda_status(e, "line trace");

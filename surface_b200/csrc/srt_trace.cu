@@ -32,6 +32,7 @@
 #include <type_traits>
 
 #include "srt_internal.cuh"
+#include "srt_packed.cuh"
 #include "srt_walks.cuh"
 
 namespace srt {
@@ -747,25 +748,6 @@ struct SharedStack {
   __shared__ uint2 NAME##_e[kShDepth][NT];                 \
   __shared__ float NAME##_t[kShDepth][NT];                 \
   SharedStack<NT> NAME(NAME##_e, NAME##_t)
-
-// Two floats as one 64-bit operand of the packed instructions: each half is
-// added and multiplied with its own IEEE rounding.
-__device__ __forceinline__ float2 add2(float2 a, float2 b) {
-  unsigned long long r;
-  asm("add.rn.f32x2 %0, %1, %2;"
-      : "=l"(r)
-      : "l"(*reinterpret_cast<unsigned long long *>(&a)),
-        "l"(*reinterpret_cast<unsigned long long *>(&b)));
-  return *reinterpret_cast<float2 *>(&r);
-}
-__device__ __forceinline__ float2 mul2(float2 a, float2 b) {
-  unsigned long long r;
-  asm("mul.rn.f32x2 %0, %1, %2;"
-      : "=l"(r)
-      : "l"(*reinterpret_cast<unsigned long long *>(&a)),
-        "l"(*reinterpret_cast<unsigned long long *>(&b)));
-  return *reinterpret_cast<float2 *>(&r);
-}
 
 // A component the slab test's products can turn into NaN.
 __device__ __forceinline__ bool odd_ray(const RayF &r) {
@@ -2790,7 +2772,7 @@ __device__ __forceinline__ bool elem_hit_lines(const SceneElem &e, const RayF &l
   unsigned long long nb = 0, nl = 0, nt = 0;
   const LineHit H = line_walk<LSTACK, true>(static_cast<const LNode *>(e.nodes),
                                             reinterpret_cast<const LineRec *>(e.prims),
-                                            e.aux != 0, R, nb, nl, nt);
+                                            (e.aux & 1) != 0, (e.aux & 2) != 0, R, nb, nl, nt);
   c[1] += (uint32_t)nb;
   c[2] += (uint32_t)nl;
   c[3] += (uint32_t)nt;
