@@ -1345,6 +1345,14 @@ constexpr size_t kWideAll = (size_t)1 << 18;
 uint32_t wide_slots(size_t n) {
   return (uint32_t)std::max<size_t>(std::min(n - 1, kWideAll), (n - 1) / 6);
 }
+// The two-child nodes and behind them, on a line of their own, the wide_cap
+// wide nodes: one allocation (a second one took as long as a small build).
+cudaError_t ensure_nodes2(srt_accel *a, size_t nodes) {
+  const size_t off = (nodes * sizeof(Node2) + 127) & ~(size_t)127;
+  const cudaError_t e = a->nodes.ensure(off + (size_t)a->wide_cap * 4 * sizeof(WideRec));
+  a->wide = e == cudaSuccess ? reinterpret_cast<WideRec *>(a->nodes.as<char>() + off) : nullptr;
+  return e;
+}
 // Wide nodes of an emitted tree (nbranches: a device word) over m internal
 // Karras nodes.
 srt_status build_wide(srt_ctx *ctx, const Node2 *nodes, const uint32_t *nbranches, size_t m,
@@ -1373,11 +1381,13 @@ srt_status build_kind(srt_accel *a, const float *v, const uint32_t *f,
   ENSURE(a->prims, n * sizeof(float4) * PrimTraits<KIND>::kCacheF4);
   ENSURE(a->scene, sizeof(SceneInfo));
   size_t max_nodes = (KIND == SRT_TETRAHEDRA) ? (2 * m + 1) : m;
-  ENSURE(a->nodes, max_nodes * (KIND == SRT_TETRAHEDRA ? sizeof(NodeT) : sizeof(Node2)));
-  if (KIND != SRT_TETRAHEDRA) {
+  if (KIND == SRT_TETRAHEDRA) {
+    ENSURE(a->nodes, max_nodes * sizeof(NodeT));
+  } else {
     a->wide_cap = wide_slots(n);
     a->wide_all = a->wide_cap >= m;
-    ENSURE(a->wide, (size_t)a->wide_cap * 4 * sizeof(WideRec));
+    if ((e = ensure_nodes2(a, max_nodes)) != cudaSuccess)
+      return cuda_status(e, "build allocation a->nodes");
   }
 
   ENSURE(ctx->s_kchild, m * 4);
@@ -1468,7 +1478,7 @@ srt_status build_kind(srt_accel *a, const float *v, const uint32_t *f,
                                                    ctx->d_err);
     ctx->launches++;
     s = build_wide(ctx, a->nodes.as<Node2>(), &scene->nbranches, m, a->wide_cap,
-                   a->wide.as<WideRec>(), &scene->irregular);
+                   a->wide, &scene->irregular);
     if (s != SRT_OK) return s;
   }
 #undef ENSURE2
@@ -2007,11 +2017,14 @@ srt_status load_kind(srt_accel *a, const float *v, const uint32_t *f, const floa
   cudaStream_t st = ctx->stream;
   cudaError_t e;
   const size_t node_bytes = (KIND == SRT_TETRAHEDRA) ? sizeof(NodeT) : sizeof(Node2);
+  a->wide_cap = KIND == SRT_TETRAHEDRA ? 0 : nbranches;
+  a->wide_all = true;
   if ((e = a->codes.ensure(n * 4)) != cudaSuccess ||
       (e = a->indices.ensure(n * 4)) != cudaSuccess ||
       (e = a->prims.ensure(n * sizeof(float4) * PrimTraits<KIND>::kCacheF4)) != cudaSuccess ||
       (e = a->scene.ensure(sizeof(SceneInfo))) != cudaSuccess ||
-      (e = a->nodes.ensure(nnodes * node_bytes)) != cudaSuccess ||
+      (e = KIND == SRT_TETRAHEDRA ? a->nodes.ensure(nnodes * node_bytes)
+                                  : ensure_nodes2(a, nnodes)) != cudaSuccess ||
       (e = ctx->s_keys2.ensure(n * 4)) != cudaSuccess)
     return cuda_status(e, "load allocation");
   SceneInfo *scene = a->scene.as<SceneInfo>();
@@ -2030,12 +2043,8 @@ srt_status load_kind(srt_accel *a, const float *v, const uint32_t *f, const floa
   set_branches_kernel<<<1, 1, 0, st>>>(scene, nbranches);
   ctx->launches += 3;
   if (KIND != SRT_TETRAHEDRA) {
-    a->wide_cap = nbranches;
-    a->wide_all = true;
-    if ((e = a->wide.ensure((size_t)nbranches * 4 * sizeof(WideRec))) != cudaSuccess)
-      return cuda_status(e, "load allocation");
     s = build_wide(ctx, a->nodes.as<Node2>(), &scene->nbranches, nbranches, nbranches,
-                   a->wide.as<WideRec>(), &scene->irregular);
+                   a->wide, &scene->irregular);
     if (s != SRT_OK) return s;
   }
   if ((e = cudaGetLastError()) != cudaSuccess) return cuda_status(e, "load");

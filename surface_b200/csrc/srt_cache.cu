@@ -289,7 +289,7 @@ bool same_key(const srt_cache_key &a, const srt_cache_key &b) {
 
 // Device bytes an accel holds (tree, order, codes, primitive cache, staging).
 uint64_t accel_bytes(const srt_accel *a) {
-  return a->nodes.cap + a->indices.cap + a->codes.cap + a->prims.cap + a->scene.cap + a->wide.cap +
+  return a->nodes.cap + a->indices.cap + a->codes.cap + a->prims.cap + a->scene.cap +
          a->in_verts.cap + a->in_faces.cap + a->in_radius.cap;
 }
 

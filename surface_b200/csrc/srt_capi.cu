@@ -326,7 +326,7 @@ SRT_API srt_status srt_accel_destroy(srt_accel *a) {
   if (!a) return SRT_OK;
   cudaSetDevice(a->ctx->device);
   cudaStreamSynchronize(a->ctx->stream);
-  DevBuf *bufs[] = {&a->nodes, &a->indices, &a->codes, &a->prims, &a->scene, &a->wide,
+  DevBuf *bufs[] = {&a->nodes, &a->indices, &a->codes, &a->prims, &a->scene,
                     &a->in_verts, &a->in_faces, &a->in_radius};
   for (DevBuf *b : bufs) b->release();
   delete a;

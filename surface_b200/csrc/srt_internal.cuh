@@ -211,7 +211,7 @@ struct srt_accel {
   // wide nodes of the tree's first wide_cap branches (a tree with more
   // branches is walked by its two-child nodes alone); wide_all: it has none
   // beyond them whatever its shape
-  srt::DevBuf wide;
+  srt::WideRec *wide = nullptr;  // behind the two-child nodes
   uint32_t wide_cap = 0;
   bool wide_all = false;
   srt::DevBuf in_verts, in_faces, in_radius;  // device copies of host inputs

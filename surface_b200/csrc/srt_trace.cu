@@ -2088,7 +2088,7 @@ static void launch_wide(srt_accel *a, const srt_ray *rays, size_t n, srt_hit *hi
   const auto kern = a->kind == SRT_TRIANGLES ? trace_wide_kernel<SRT_TRIANGLES>
                                              : trace_wide_kernel<SRT_SPHERES>;
   kern<<<(unsigned)((n + 31) / 32), 128, 0, ctx->stream>>>(
-      a->wide.as<WideRec>(), a->wide_cap, a->nodes.as<Node2>(), a->prims.as<float4>(),
+      a->wide, a->wide_cap, a->nodes.as<Node2>(), a->prims.as<float4>(),
       a->indices.as<uint32_t>(), rays, n, hits, a->scene.as<SceneInfo>(), prev_normals,
       normal_out, stats, dlist, dcount, max_iter, ctx->d_err, order);
   ctx->launches++;
