@@ -6,8 +6,9 @@
 // traversal (timed with CUDA events, one axis at a time from the default
 // point): block size x rays per grab, then the traversal stack depth (24, 32
 // or 48 entries; a depth the trees overflow is dropped), then the ray order
-// (array order, or sorted within each scene by the top 12 or 22 bits of a
-// Morton code over origin and direction, the sort timed with the trace).
+// (tiles of the rays' rows, or sorted within each scene by the top 12 or 22
+// bits of a Morton code over origin and direction, the sort timed with the
+// trace).
 // The second identical call captures the whole sequence in a CUDA graph,
 // later identical calls replay it with one graph launch.
 #include <cstring>
@@ -78,7 +79,9 @@ srt_status trace_tuned(srt_batch *b, int block, int R, int depth, int sort_bits)
   const size_t n = b->bt.nrays;
   cudaError_t e;
   if (sort_bits == 0) {  // the scenes' rays in tiles of their rows
-    if ((e = b->rorder.ensure(n * 4)) != cudaSuccess) return cuda_status(e, "batch ray order");
+    if (b->rorder.ensure(n * 4) != cudaSuccess)  // array order does as well
+      return launch_trace_batch(b->ctx, b->bt, b->rays, b->hits, block, R, nullptr, depth,
+                                nullptr);
     srt_status s = raster_order(b->ctx, b->rays, n, b->bt.roff.as<uint32_t>(), b->bt.nseg,
                                 b->rorder.as<uint32_t>());
     if (s != SRT_OK) return s;
@@ -114,7 +117,7 @@ srt_status take_limit_flag(srt_ctx *ctx, bool &hit) {
 }
 
 // Time the traversal over the tuning axes, one at a time from the default
-// point (block 128, one grab of 32 rays, depth 32, array order), and keep
+// point (block 128, one grab of 32 rays, depth 32, tiles of rows), and keep
 // the fastest point.
 srt_status autotune(srt_batch *b) {
   static const int blocks[] = {64, 128, 256};

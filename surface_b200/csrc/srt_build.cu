@@ -1347,9 +1347,15 @@ uint32_t wide_slots(size_t n) {
 }
 // The two-child nodes and behind them, on a line of their own, the wide_cap
 // wide nodes: one allocation (a second one took as long as a small build).
+// Without memory for the wide ones the two-child nodes are walked.
 cudaError_t ensure_nodes2(srt_accel *a, size_t nodes) {
   const size_t off = (nodes * sizeof(Node2) + 127) & ~(size_t)127;
-  const cudaError_t e = a->nodes.ensure(off + (size_t)a->wide_cap * 4 * sizeof(WideRec));
+  cudaError_t e = a->nodes.ensure(off + (size_t)a->wide_cap * 4 * sizeof(WideRec));
+  if (e == cudaErrorMemoryAllocation) {
+    a->wide_cap = 0;
+    a->wide_all = false;
+    e = a->nodes.ensure(off);
+  }
   a->wide = e == cudaSuccess ? reinterpret_cast<WideRec *>(a->nodes.as<char>() + off) : nullptr;
   return e;
 }

@@ -272,8 +272,8 @@ srt_status raster_order(srt_ctx *ctx, const srt_ray *rays, size_t n, const uint3
 }
 
 srt_status raster_order(srt_ctx *ctx, const srt_ray *rays, size_t n, const uint32_t **order) {
-  cudaError_t e = ctx->s_rorder.ensure(n * 4);
-  if (e != cudaSuccess) return cuda_status(e, "ray order scratch");
+  *order = nullptr;
+  if (ctx->s_rorder.ensure(n * 4) != cudaSuccess) return SRT_OK;  // array order does as well
   *order = ctx->s_rorder.as<uint32_t>();
   return raster_order(ctx, rays, n, nullptr, 1, ctx->s_rorder.as<uint32_t>());
 }

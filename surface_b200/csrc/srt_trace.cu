@@ -2058,6 +2058,7 @@ resolve_batch_kernel(const Node2 *__restrict__ nodes, const float4 *__restrict__
 // 512^2 318 / 303, 1400^2 1110 / 1018; spheres 100,000: 512^2 204 / 188,
 // 1400^2 771 / 633.
 bool takes_tiles(const srt_accel *a, size_t n) {
+  if (n >= (size_t)1 << 32) return false;
   if (a->kind == SRT_TETRAHEDRA) return n >= (size_t)1 << 16;
   return n >= (size_t)1 << (a->n < ((size_t)1 << 15) ? 20 : 18);
 }

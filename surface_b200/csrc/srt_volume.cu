@@ -781,9 +781,10 @@ SRT_API srt_status srt_volume_march_fwd_ex(srt_ctx *ctx, const srt_volume_params
   if (samples >= kBrickSamples + 4.0 * (double)nvox * kBrickTexel && params->alpha_max >= 0.0f &&
       std::isfinite(params->sigma_scale) && std::isfinite(params->step) && nb.y < 65536 &&
       nb.z < 65536) {
-    if ((e = ctx->s_brick.ensure((size_t)nb.x * nb.y * nb.z)) != cudaSuccess)
-      return cuda_status(e, "volume bricks");
-    occ = ctx->s_brick.as<uint8_t>();
+    if (ctx->s_brick.ensure((size_t)nb.x * nb.y * nb.z) == cudaSuccess)
+      occ = ctx->s_brick.as<uint8_t>();
+  }
+  if (occ) {
     vol_brick_kernel<<<dim3((unsigned)(nb.x + 31) / 32, nb.y, nb.z), 288, 0, st>>>(
         static_cast<const float *>(dd), dim, nb, static_cast<const float4 *>(dt), tf_entries, occ);
     ctx->launches++;
