@@ -335,6 +335,7 @@ struct SceneWork {
   uint32_t max_iter;
   unsigned long long *stats;
   uint32_t *err;
+  const uint32_t *order;  // the keys' p-th ray is order[p]; NULL: ray p
 };
 // Side streams of a scene's trace: one per element kind and one for the
 // rays with more candidates than slots, forked from and joined to the
