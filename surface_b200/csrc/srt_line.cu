@@ -17,10 +17,10 @@
 // rays' rows or a Morton order for large batches), in the reference's order
 // (a branch's box against the closest hit so far, then its near and its far
 // child by the sign of the ray's direction on the branch's axis), every line
-// of an entered leaf tested in order by CylinderIsect (:488-577).  Compiled without FMA contraction; the
-// reference's unqualified sqrt and fabs are the double C functions, so the
-// quadratic's first root is formed in double, and every other sqrt and
-// reciprocal rounds as the float operation does.
+// of an entered leaf tested in order by CylinderIsect (:488-577).  Compiled
+// without FMA contraction; the reference's unqualified sqrt and fabs are the
+// double C functions, so the quadratic's first root is formed in double, and
+// every other sqrt and reciprocal rounds as the float operation does.
 #include <algorithm>
 #include <cmath>
 #include <cstdio>
@@ -578,8 +578,8 @@ template <int STACK, bool STATS>
 __global__ void __launch_bounds__(128, STACK <= 64 ? 8 : 1)
 line_trace_kernel(const LNode *__restrict__ nodes, const LineRec *__restrict__ recs, bool cap,
                   bool ordered, const srt_ray *__restrict__ rays,
-                  const uint32_t *__restrict__ order, size_t n, srt_hit *__restrict__ hits, float *__restrict__ normals,
-                  unsigned long long *__restrict__ stats) {
+                  const uint32_t *__restrict__ order, size_t n, srt_hit *__restrict__ hits,
+                  float *__restrict__ normals, unsigned long long *__restrict__ stats) {
   unsigned long long nb = 0, nl = 0, nt = 0;
   for (size_t k = blockIdx.x * (size_t)blockDim.x + threadIdx.x; k < n;
        k += (size_t)gridDim.x * blockDim.x) {
@@ -761,7 +761,8 @@ SRT_API srt_status srt_line_build(srt_line_accel *a, const float *positions, siz
       (e = grow(bsum, ((size_t)tiles + 1) * 4)) != cudaSuccess ||
       (e = grow(cnt, 16)) != cudaSuccess)
     return cuda_status(e, "line build scratch");
-  uint32_t *d_err = cnt.as<uint32_t>(), *d_pairs = d_err + 1, *d_next = d_err + 2, *d_bad = d_err + 3;
+  uint32_t *d_err = cnt.as<uint32_t>(), *d_pairs = d_err + 1, *d_next = d_err + 2,
+           *d_bad = d_err + 3;
   cudaMemsetAsync(d_err, 0, 16, st);
   const unsigned egrid = (unsigned)std::min<size_t>((n + 255) / 256, (size_t)ctx->num_sms * 16);
   line_prep_kernel<<<egrid, 256, 0, st>>>(
@@ -931,18 +932,13 @@ SRT_API srt_status srt_line_trace(srt_line_accel *a, const srt_ray *rays, size_t
   const uint32_t *ord = nullptr;
   if (n >= 32768 && (s = ray_order(ctx, rr, n, &ord)) != SRT_OK) return s;
   const bool shallow = a->depth + 2 <= 64;
-  if (shallow && !st)
-    line_trace_kernel<64, false><<<grid, 128, 0, ctx->stream>>>(nd, rc, a->cap, a->ordered, rr, ord, n, dh,
-                                                                 dn, st);
-  else if (shallow)
-    line_trace_kernel<64, true><<<grid, 128, 0, ctx->stream>>>(nd, rc, a->cap, a->ordered, rr, ord, n, dh,
-                                                                dn, st);
-  else if (!st)
-    line_trace_kernel<520, false><<<grid, 128, 0, ctx->stream>>>(nd, rc, a->cap, a->ordered, rr, ord, n, dh,
-                                                                  dn, st);
+  auto launch = [&](auto kernel) {
+    kernel<<<grid, 128, 0, ctx->stream>>>(nd, rc, a->cap, a->ordered, rr, ord, n, dh, dn, st);
+  };
+  if (shallow)
+    st ? launch(line_trace_kernel<64, true>) : launch(line_trace_kernel<64, false>);
   else
-    line_trace_kernel<520, true><<<grid, 128, 0, ctx->stream>>>(nd, rc, a->cap, a->ordered, rr, ord, n, dh,
-                                                                 dn, st);
+    st ? launch(line_trace_kernel<520, true>) : launch(line_trace_kernel<520, false>);
   ctx->launches++;
   if ((e = cudaGetLastError()) != cudaSuccess) return cuda_status(e, "line trace");
   if (!hdev) cudaMemcpyAsync(hits, dh, n * sizeof(srt_hit), cudaMemcpyDeviceToHost, ctx->stream);
