@@ -2917,7 +2917,7 @@ void scene_occupancy() {
 // element's items as well: a warp's 32 rays of an element lie in a square of
 // the image.  Measured, array order / tiles, us: 64 elements 1024^2 2983 /
 // 2632, 860^2 2323 / 2227, 512^2 1296 / 1231; 8 elements 1024^2 1429 / 1386,
-// 860^2 1204 / 1247, 512^2 827 / 933; 3 elements 1024^2 675 / 635, 512^2
+// 860^2 1204 / 1247, 512^2 827 / 933; one element 1024^2 675 / 635, 512^2
 // 492 / 502, 256^2 385 / 423 -- smaller images wait for the launches, not for
 // divergence.
 constexpr size_t kSceneTiles = (size_t)1 << 20;
