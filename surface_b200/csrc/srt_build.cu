@@ -1385,7 +1385,9 @@ cudaError_t ensure_nodes2(srt_accel *a, size_t nodes) {
     a->wide_all = false;
     e = a->nodes.ensure(off);
   }
-  a->wide = e == cudaSuccess ? reinterpret_cast<WideRec *>(a->nodes.as<char>() + off) : nullptr;
+  a->wide = e == cudaSuccess && a->wide_cap
+                ? reinterpret_cast<WideRec *>(a->nodes.as<char>() + off)
+                : nullptr;
   return e;
 }
 // Wide nodes of an emitted tree (nbranches: a device word) over m internal
@@ -2087,7 +2089,7 @@ srt_status load_kind(srt_accel *a, const float *v, const uint32_t *f, const floa
   set_branches_kernel<<<1, 1, 0, st>>>(scene, nbranches);
   ctx->launches += 3;
   if (KIND != SRT_TETRAHEDRA) {
-    s = build_wide(ctx, a->nodes.as<Node2>(), &scene->nbranches, nbranches, nbranches,
+    s = build_wide(ctx, a->nodes.as<Node2>(), &scene->nbranches, nbranches, a->wide_cap,
                    a->wide, &scene->irregular);
     if (s != SRT_OK) return s;
   }
