@@ -232,6 +232,23 @@ SRT_API const char *srt_last_error(void) { return g_last_error.c_str(); }
 
 SRT_API uint64_t srt_ctx_launch_count(srt_ctx *ctx) { return ctx ? ctx->launches : 0; }
 
+// A pool that keeps up to 64 MB between calls (it grows in blocks of some 32;
+// the largest call takes 4).
+static cudaMemPool_t make_pool(int device) {
+  cudaMemPoolProps props = {};
+  props.allocType = cudaMemAllocationTypePinned;
+  props.location.type = cudaMemLocationTypeDevice;
+  props.location.id = device;
+  cudaMemPool_t pool = nullptr;
+  uint64_t keep = (uint64_t)64 << 20;
+  if (cudaMemPoolCreate(&pool, &props) != cudaSuccess) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep);
+  return pool;
+}
+
 SRT_API srt_status srt_ctx_create(int device, srt_ctx **out) {
   if (!out) return SRT_ERR_INVALID;
   *out = nullptr;
@@ -263,6 +280,7 @@ SRT_API srt_status srt_ctx_create(int device, srt_ctx **out) {
   }
   cudaMemset(c->d_err, 0, 4);
   *c->h_err = 0;
+  c->pool = make_pool(device);
   *out = c;
   return SRT_OK;
 }
@@ -278,14 +296,15 @@ SRT_API srt_status srt_ctx_destroy(srt_ctx *c) {
                     &c->s_stage_scal, &c->s_stage_norm, &c->s_defer, &c->s_spawn, &c->s_rkey,
                     &c->s_rorder, &c->s_isect_sub, &c->s_stage_isect, &c->s_keys3,
                     &c->s_vals3, &c->s_status, &c->s_lscan, &c->s_rays_in,
-                    &c->s_kidx, &c->s_kprefix, &c->s_raster, &c->s_brick,
-                    &c->s_status_lg};
+                    &c->s_kidx, &c->s_kprefix, &c->s_raster, &c->s_status_lg};
   if (c->copy_stream) cudaStreamSynchronize(c->copy_stream);
   for (DevBuf *b : bufs) b->release();
   if (c->ev_copy) cudaEventDestroy(c->ev_copy);
   if (c->ev_inputs) cudaEventDestroy(c->ev_inputs);
   if (c->ev_free) cudaEventDestroy(c->ev_free);
   if (c->copy_stream) cudaStreamDestroy(c->copy_stream);
+  // (what a call under way on another stream holds of it goes when that ends)
+  if (c->pool) cudaMemPoolDestroy(c->pool);
   if (c->d_err) cudaFree(c->d_err);
   if (c->h_err) cudaFreeHost(c->h_err);
   if (c->own_stream) cudaStreamDestroy(c->own_stream);

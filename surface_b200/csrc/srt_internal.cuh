@@ -187,7 +187,10 @@ struct srt_ctx {
       s_kparent, s_counter, s_ibox, s_flag, s_slot, s_partial,
       s_stage_in, s_stage_out, s_stage_aux, s_stage_sub, s_stage_scal, s_stage_norm,
       s_defer, s_spawn, s_rkey, s_rorder, s_isect_sub, s_stage_isect, s_keys3, s_vals3,
-      s_status, s_lscan, s_rays_in, s_kidx, s_kprefix, s_raster, s_brick, s_status_lg;
+      s_status, s_lscan, s_rays_in, s_kidx, s_kprefix, s_raster, s_status_lg;
+  // memory of single calls, taken and given back in the order of the call's
+  // stream (vol_brick_kernel's marks); NULL where the device has no such pools
+  cudaMemPool_t pool = nullptr;
   uint32_t os_epoch = 0;  // look-back epoch of the last sort pass (srt_sort.cu)
   // recorded after a build's host inputs were copied; the next staged ray
   // array waits for it (inputs_pending)

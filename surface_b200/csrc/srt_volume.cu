@@ -780,9 +780,14 @@ SRT_API srt_status srt_volume_march_fwd_ex(srt_ctx *ctx, const srt_volume_params
       (double)npix * std::min<double>(params->max_steps, 2.0 / (double)params->step);
   if (samples >= kBrickSamples + 4.0 * (double)nvox * kBrickTexel && params->alpha_max >= 0.0f &&
       std::isfinite(params->sigma_scale) && std::isfinite(params->step) && nb.y < 65536 &&
-      nb.z < 65536) {
-    if (ctx->s_brick.ensure((size_t)nb.x * nb.y * nb.z) == cudaSuccess)
-      occ = ctx->s_brick.as<uint8_t>();
+      nb.z < 65536 && ctx->pool) {
+    // the call's own marks, in its stream's order: marches may run at the same
+    // time on several streams, and under capture they belong to the graph
+    if (cudaMallocFromPoolAsync(reinterpret_cast<void **>(&occ), (size_t)nb.x * nb.y * nb.z,
+                                ctx->pool, st) != cudaSuccess) {
+      cudaGetLastError();
+      occ = nullptr;  // every sample is marched
+    }
   }
   if (occ) {
     vol_brick_kernel<<<dim3((unsigned)(nb.x + 31) / 32, nb.y, nb.z), 288, 0, st>>>(
@@ -800,7 +805,9 @@ SRT_API srt_status srt_volume_march_fwd_ex(srt_ctx *ctx, const srt_volume_params
       K, static_cast<const float *>(dd), static_cast<const float4 *>(dt),
       reinterpret_cast<float4 *>(di), dtr, occ, nb);
   ctx->launches++;
-  if ((e = cudaGetLastError()) != cudaSuccess) return cuda_status(e, "volume fwd");
+  e = cudaGetLastError();
+  if (occ) cudaFreeAsync(occ, st);
+  if (e != cudaSuccess) return cuda_status(e, "volume fwd");
   if (!img_dev) cudaMemcpyAsync(image, di, npix * 16, cudaMemcpyDeviceToHost, st);
   if (!tr_dev) cudaMemcpyAsync(transmittance, dtr, npix * 4, cudaMemcpyDeviceToHost, st);
   const bool staged = remap_tmp[0].p || remap_tmp[1].p || remap_tmp[2].p;
