@@ -34,6 +34,10 @@ struct VolConst {
   int clamp[3];
 };
 
+__device__ __forceinline__ float wrap_coord(const VolConst &K, int k, float u) {
+  return K.clamp[k] ? u : u - (float)floor_ref(u);
+}
+
 // The fetch coordinate of axis k: local::remap (gles/gles_common.h:264-269)
 // then the repeat wrap of FilterTexture3DFloat unless clamp-to-edge.
 __device__ __forceinline__ float tex_coord(const VolConst &K, int k, float u) {
@@ -43,8 +47,7 @@ __device__ __forceinline__ float tex_coord(const VolConst &K, int k, float u) {
     idx = max(min(nk - 1, idx), 0);
     u = __ldg(&K.remap[k][idx]);
   }
-  if (!K.clamp[k]) u = u - (float)floor_ref(u);
-  return u;
+  return wrap_coord(K, k, u);
 }
 
 // Lower texel corner (clamped) and trilinear fractions of a fetch.
@@ -206,8 +209,12 @@ constexpr int kTfMax = 1024;  // longest transfer function (vol_bwd_kernel's sha
 // share their coordinates / 8; it is empty when every table entry that a
 // density between the smallest and largest of its 9^3 texels can reach has
 // opacity 0 (and a finite colour, so that 0 times it is 0).
+// A remap table's values may leave [0, 1] or be NaN: the fetch then takes an
+// edge texel (the first for NaN) and does not interpolate, so the outermost
+// bricks of that side count as full.
 constexpr int kBrickShift = 3;
 constexpr int kBrick = 1 << kBrickShift;
+constexpr int kTableLook = 4096;  // longer tables are taken to have such values unseen
 
 // occ[brick] = 0 for an empty brick.  A block takes 32 bricks of a row: a
 // thread per texel column, 81 texels each, coalesced along x; the smallest
@@ -215,8 +222,10 @@ constexpr int kBrick = 1 << kBrickShift;
 // reading the density once: 67 MB in 29 us (44 us while each row's load waited
 // for a bounds test).
 __global__ void __launch_bounds__(288)
-vol_brick_kernel(const float *__restrict__ dens, int3 dim, int3 nb, const float4 *__restrict__ tf,
-                 int tfn, uint8_t *__restrict__ occ) {
+vol_brick_kernel(const VolConst K, const float *__restrict__ dens, int3 nb,
+                 const float4 *__restrict__ tf, uint8_t *__restrict__ occ) {
+  const int3 dim = make_int3(K.dim[0], K.dim[1], K.dim[2]);
+  const int tfn = K.tfn;
   __shared__ float s_min[kBrick * 32 + 1], s_max[kBrick * 32 + 1];
   __shared__ uint32_t s_bad[kTfMax + 1];  // entries that are not transparent, before each
   const int x0 = blockIdx.x * kBrick * 32, by = blockIdx.y, bz = blockIdx.z;
@@ -235,6 +244,24 @@ vol_brick_kernel(const float *__restrict__ dens, int3 dim, int3 nb, const float4
       run += __popc(m);
     }
     if (threadIdx.x == 0) s_bad[tfn] = run;
+  }
+  // sides of the volume on which a remap table reaches past it
+  bool below[3] = {}, above[3] = {};
+  const int first[3] = {(int)blockIdx.x * 32, by, bz};
+  const int last[3] = {min(first[0] + 31, nb.x - 1), by, bz}, sides[3] = {nb.x, nb.y, nb.z};
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    const int n = K.nremap[k];
+    if (!n || (first[k] > 0 && last[k] < sides[k] - 1)) continue;
+    bool lo = n > kTableLook, hi = lo;
+    if (!lo)
+      for (int i = (int)threadIdx.x; i < n; i += (int)blockDim.x) {
+        const float u = wrap_coord(K, k, __ldg(&K.remap[k][i]));
+        lo = lo || !(u >= 0.0f);
+        hi = hi || u > 1.0f;
+      }
+    below[k] = __syncthreads_or(lo);
+    above[k] = __syncthreads_or(hi);
   }
   const int col = (int)threadIdx.x;
   if (col <= kBrick * 32) {
@@ -277,6 +304,10 @@ vol_brick_kernel(const float *__restrict__ dens, int3 dim, int3 nb, const float4
     const int i0 = max((int)a - 1, 0), i1 = min((int)c + 3, tfn);  // [i0, i1)
     full = s_bad[i1] != s_bad[i0];
   }
+  const int at[3] = {bx, by, bz};
+#pragma unroll
+  for (int k = 0; k < 3; k++)
+    full = full || (below[k] && at[k] == 0) || (above[k] && at[k] == sides[k] - 1);
   occ[((size_t)bz * nb.y + by) * nb.x + bx] = full ? 1 : 0;
 }
 
@@ -772,7 +803,6 @@ SRT_API srt_status srt_volume_march_fwd_ex(srt_ctx *ctx, const srt_volume_params
   const size_t nthreads = (size_t)((params->width + 7) / 8) * ((params->height + 3) / 4) * 32;
   // bricks: when the march is long enough to gain from them (they cost one
   // reading of the density and 5 us) and a transparent sample's alpha is 0
-  const int3 dim = make_int3(dims[0], dims[1], dims[2]);
   const int3 nb = make_int3((dims[0] + kBrick - 1) / kBrick, (dims[1] + kBrick - 1) / kBrick,
                             (dims[2] + kBrick - 1) / kBrick);
   uint8_t *occ = nullptr;
@@ -791,7 +821,7 @@ SRT_API srt_status srt_volume_march_fwd_ex(srt_ctx *ctx, const srt_volume_params
   }
   if (occ) {
     vol_brick_kernel<<<dim3((unsigned)(nb.x + 31) / 32, nb.y, nb.z), 288, 0, st>>>(
-        static_cast<const float *>(dd), dim, nb, static_cast<const float4 *>(dt), tf_entries, occ);
+        K, static_cast<const float *>(dd), nb, static_cast<const float4 *>(dt), occ);
     ctx->launches++;
   }
   bool plain = true;
