@@ -803,14 +803,15 @@ SRT_API srt_status srt_volume_march_fwd_ex(srt_ctx *ctx, const srt_volume_params
   const size_t nthreads = (size_t)((params->width + 7) / 8) * ((params->height + 3) / 4) * 32;
   // bricks: when the march is long enough to gain from them (they cost one
   // reading of the density and 5 us) and a transparent sample's alpha is 0
-  const int3 nb = make_int3((dims[0] + kBrick - 1) / kBrick, (dims[1] + kBrick - 1) / kBrick,
-                            (dims[2] + kBrick - 1) / kBrick);
+  const int3 nb = make_int3((dims[0] - 1) / kBrick + 1, (dims[1] - 1) / kBrick + 1,
+                            (dims[2] - 1) / kBrick + 1);
   uint8_t *occ = nullptr;
   const double samples =
       (double)npix * std::min<double>(params->max_steps, 2.0 / (double)params->step);
   if (samples >= kBrickSamples + 4.0 * (double)nvox * kBrickTexel && params->alpha_max >= 0.0f &&
       std::isfinite(params->sigma_scale) && std::isfinite(params->step) && nb.y < 65536 &&
-      nb.z < 65536 && ctx->pool) {
+      nb.z < 65536 && dims[0] <= (1 << 30) &&  // (texels past a row's end in 32 bits)
+      ctx->pool) {
     // the call's own marks, in its stream's order: marches may run at the same
     // time on several streams, and under capture they belong to the graph
     if (cudaMallocFromPoolAsync(reinterpret_cast<void **>(&occ), (size_t)nb.x * nb.y * nb.z,
