@@ -1374,17 +1374,22 @@ constexpr size_t kWideAll = (size_t)1 << 18;
 uint32_t wide_slots(size_t n) {
   return (uint32_t)std::max<size_t>(std::min(n - 1, kWideAll), (n - 1) / 6);
 }
-// The two-child nodes and behind them, on a line of their own, the wide_cap
-// wide nodes: one allocation (a second one took as long as a small build).
+// Room for `nodes` two-child nodes and behind them, on a line of their own,
+// `slots` wide nodes: one allocation (a second one took as long as a small
+// build).  A buffer that holds the two-child nodes is kept as it is laid out.
 // Without memory for the wide ones the two-child nodes are walked.
-cudaError_t ensure_nodes2(srt_accel *a, size_t nodes) {
+cudaError_t ensure_nodes2(srt_accel *a, size_t nodes, uint32_t slots) {
+  if (a->nodes.p && nodes <= a->node_cap) return cudaSuccess;
+  a->nodes.release();
   const size_t off = (nodes * sizeof(Node2) + 127) & ~(size_t)127;
-  cudaError_t e = a->nodes.ensure(off + (size_t)a->wide_cap * 4 * sizeof(WideRec));
+  a->wide_cap = slots;
+  cudaError_t e = a->nodes.ensure(off + (size_t)slots * 4 * sizeof(WideRec));
   if (e == cudaErrorMemoryAllocation) {
     a->wide_cap = 0;
-    a->wide_all = false;
     e = a->nodes.ensure(off);
   }
+  a->node_cap = e == cudaSuccess ? nodes : 0;
+  a->wide_all = a->wide_cap >= nodes;
   a->wide = e == cudaSuccess && a->wide_cap
                 ? reinterpret_cast<WideRec *>(a->nodes.as<char>() + off)
                 : nullptr;
@@ -1421,9 +1426,7 @@ srt_status build_kind(srt_accel *a, const float *v, const uint32_t *f,
   if (KIND == SRT_TETRAHEDRA) {
     ENSURE(a->nodes, max_nodes * sizeof(NodeT));
   } else {
-    a->wide_cap = wide_slots(n);
-    a->wide_all = a->wide_cap >= m;
-    if ((e = ensure_nodes2(a, max_nodes)) != cudaSuccess)
+    if ((e = ensure_nodes2(a, max_nodes, wide_slots(n))) != cudaSuccess)
       return cuda_status(e, "build allocation a->nodes");
   }
 
@@ -2063,14 +2066,12 @@ srt_status load_kind(srt_accel *a, const float *v, const uint32_t *f, const floa
   cudaStream_t st = ctx->stream;
   cudaError_t e;
   const size_t node_bytes = (KIND == SRT_TETRAHEDRA) ? sizeof(NodeT) : sizeof(Node2);
-  a->wide_cap = KIND == SRT_TETRAHEDRA ? 0 : nbranches;
-  a->wide_all = true;
   if ((e = a->codes.ensure(n * 4)) != cudaSuccess ||
       (e = a->indices.ensure(n * 4)) != cudaSuccess ||
       (e = a->prims.ensure(n * sizeof(float4) * PrimTraits<KIND>::kCacheF4)) != cudaSuccess ||
       (e = a->scene.ensure(sizeof(SceneInfo))) != cudaSuccess ||
       (e = KIND == SRT_TETRAHEDRA ? a->nodes.ensure(nnodes * node_bytes)
-                                  : ensure_nodes2(a, nnodes)) != cudaSuccess ||
+                                  : ensure_nodes2(a, nnodes, nbranches)) != cudaSuccess ||
       (e = ctx->s_keys2.ensure(n * 4)) != cudaSuccess)
     return cuda_status(e, "load allocation");
   SceneInfo *scene = a->scene.as<SceneInfo>();

@@ -208,13 +208,15 @@ struct srt_accel {
   srt_ctx *ctx = nullptr;
   srt_kind kind = SRT_TRIANGLES;
   size_t n = 0;
-  size_t nnodes_cap = 0;
   bool built = false;
   srt::DevBuf nodes, indices, codes, prims, scene;
-  // wide nodes of the tree's first wide_cap branches (a tree with more
-  // branches is walked by its two-child nodes alone); wide_all: it has none
-  // beyond them whatever its shape
-  srt::WideRec *wide = nullptr;  // behind the two-child nodes
+  // Wide nodes of the tree's first wide_cap branches, in the nodes' buffer
+  // behind node_cap two-child nodes (a tree with more branches is walked by its
+  // two-child nodes alone); wide_all: no tree that fits has more.  All four
+  // change only when the buffer does: a trace captured in a CUDA graph stays
+  // valid over rebuilds that fit.
+  srt::WideRec *wide = nullptr;
+  size_t node_cap = 0;
   uint32_t wide_cap = 0;
   bool wide_all = false;
   srt::DevBuf in_verts, in_faces, in_radius;  // device copies of host inputs
