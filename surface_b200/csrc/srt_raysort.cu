@@ -261,6 +261,7 @@ __global__ void raster_fill_kernel(size_t n, const uint32_t *__restrict__ roff, 
 
 srt_status raster_order(srt_ctx *ctx, const srt_ray *rays, size_t n, const uint32_t *roff,
                         int nseg, uint32_t *order) {
+  if (n == 0) return SRT_OK;
   cudaError_t e = ctx->s_raster.ensure((size_t)nseg * 4);
   if (e != cudaSuccess) return cuda_status(e, "ray rows");
   uint32_t *width = ctx->s_raster.as<uint32_t>();
