@@ -1306,8 +1306,12 @@ __global__ void widen_kernel(const Node2 *__restrict__ nodes,
                              const uint32_t *__restrict__ nbranches, uint32_t cap,
                              WideRec *__restrict__ wide, uint32_t *__restrict__ irregular) {
   const uint32_t nb = *nbranches;
-  if (nb > cap) {  // the two-child nodes are walked instead, their boxes unseen
-    if (blockIdx.x == 0 && threadIdx.x == 0) *irregular = 1u;
+  if (nb > cap) {  // the two-child nodes are walked instead: a thread per child
+    for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < 2 * nb;
+         t += gridDim.x * blockDim.x) {
+      const Box2 p = node2_child(nodes[t >> 1], t & 1u);
+      if (!(p.lo[0] <= p.hi[0] && p.lo[1] <= p.hi[1] && p.lo[2] <= p.hi[2])) *irregular = 1u;
+    }
     return;
   }
   for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < 4 * nb;
@@ -1399,7 +1403,7 @@ cudaError_t ensure_nodes2(srt_accel *a, size_t nodes, uint32_t slots) {
 // Karras nodes.
 srt_status build_wide(srt_ctx *ctx, const Node2 *nodes, const uint32_t *nbranches, size_t m,
                       uint32_t cap, WideRec *wide, uint32_t *irregular) {
-  const int g = grid_for(std::min<size_t>(m, cap) / 2 + 1, kBlock, ctx->num_sms * 8);
+  const int g = grid_for(m / 2 + 1, kBlock, ctx->num_sms * 8);
   widen_kernel<<<g, kBlock, 0, ctx->stream>>>(nodes, nbranches, cap, wide, irregular);
   ctx->launches++;
   return cuda_status(cudaGetLastError(), "wide nodes");
