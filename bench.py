@@ -185,22 +185,15 @@ def profiled_traffic(kind):
     return None
 
 
-def wide_walk(kind, nrays, nprims):
-    """Whether a trace takes the walk over wide nodes (srt_trace.cu's rule)."""
-    return kind != "tet" and (nrays < 1 << 19 or (kind == "tri" and nprims >= 1 << 15))
-
-
-def algorithmic_bytes_per_ray(kind, stats, nrays, wide=False):
+def algorithmic_bytes_per_ray(kind, stats, nrays):
     """Per-ray bytes the traversal must move: ray (32) + hit (16) + nodes
-    visited x node size (two children 64, wide 128) + primitives tested x
-    primitive record."""
-    node = 128 if wide else 64
+    visited x node size + primitives tested x primitive record."""
     branch, leaf, prim = (float(x) / nrays for x in stats)
     if kind == "tet":
         return 32 + 16 + 4 + 4 + branch * 32 + prim * (48 + 4)
     if kind == "tri":
-        return 32 + 16 + branch * node + prim * 48
-    return 32 + 16 + branch * node + prim * (16 + 4)
+        return 32 + 16 + branch * 64 + prim * 48
+    return 32 + 16 + branch * 64 + prim * (16 + 4)
 
 
 # ---------------------------------------------------------------- clocks
@@ -1642,7 +1635,7 @@ def run_frame(args, W):
     e2e_ms = max_over_ranks([1e3 * sum(e2e_s) / len(e2e_s)], dev)[0]
 
     hbm, src = peaks()
-    bpr = algorithmic_bytes_per_ray("tri", stats, nr, wide_walk("tri", nr, f.shape[0]))
+    bpr = algorithmic_bytes_per_ray("tri", stats, nr)
     tr_ms = statistics.mean(t_ms)
     achieved = bpr * nr / (tr_ms * 1e-3) / 1e9
     roofline = {"bound": "hbm", "kernel": "trace", "achieved": round(achieved, 1),
@@ -1990,8 +1983,7 @@ def run_ours(args, W):
 
     # ---- roofline of the dominant kernel (traversal)
     hbm, src = peaks()
-    nprims = prims.shape[0] if prims is not None else verts.shape[0]
-    bpr = algorithmic_bytes_per_ray(kind, stats, nr, wide_walk(kind, nr, nprims))
+    bpr = algorithmic_bytes_per_ray(kind, stats, nr)
     tr_ms = statistics.mean(trace_ms)
     achieved = bpr * nr / (tr_ms * 1e-3) / 1e9
     roofline = {"bound": "hbm", "kernel": "trace", "achieved": round(achieved, 1),

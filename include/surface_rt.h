@@ -129,9 +129,10 @@ typedef struct srt_trace_opts {
    * as BuildIntersection computes it) */
   float *normal_out;
   /* work counters (device memory, 4 x uint64, accumulated): branch nodes
-   * visited (a wide node counts once), leaves visited, primitive tests -- the reference's
+   * visited, leaves visited, primitive tests -- the reference's
    * TetraTraversalStatistics (render/render_accel_tetra.h:70-78) -- and
-   * rays that took the reference's walk */
+   * rays that took the reference's walk.  They count the two-child nodes'
+   * walk, which a call with counters takes at every size. */
   unsigned long long *stats;
   /* SRT_TRACE_* bits */
   uint32_t flags;

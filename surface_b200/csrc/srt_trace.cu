@@ -1071,8 +1071,6 @@ __device__ __forceinline__ WidePass pass1_wide(const WideTree<KIND> &T, const Gr
       const uint2 rc = __ldg(reinterpret_cast<const uint2 *>(T.wide + leaf) + 3);
       j = rc.x + (uint32_t)G.lane;
       end = rc.x + rc.y;
-      w.leaf++;
-      w.prim += rc.y;
     }
     if (KIND == SRT_TRIANGLES) {
       for (; j < end; j += kGrp) {
@@ -1105,8 +1103,6 @@ __device__ __forceinline__ WidePass pass1_wide(const WideTree<KIND> &T, const Gr
     __syncwarp();
     bnd = bound_rel(G.min4(C.m), kRelTri);
   }
-  w.branch = w.it;
-  if (G.lane) w.branch = w.leaf = w.prim = 0;  // the group's work, counted once
   // merge the lanes' candidates
   WidePass r;
   const float m = G.min4(C.m);
@@ -1166,9 +1162,8 @@ trace_wide_kernel(const WideRec *__restrict__ wide, uint32_t wide_cap,
                   const uint32_t *__restrict__ sidx, const srt_ray *__restrict__ rays, size_t n,
                   srt_hit *__restrict__ hits, const SceneInfo *__restrict__ scene,
                   const float *__restrict__ prev_normals, float *__restrict__ normal_out,
-                  unsigned long long *__restrict__ stats, Deferred *__restrict__ dlist,
-                  uint32_t *__restrict__ dcount, uint32_t max_iter, uint32_t *__restrict__ err,
-                  const uint32_t *__restrict__ order) {
+                  Deferred *__restrict__ dlist, uint32_t *__restrict__ dcount, uint32_t max_iter,
+                  uint32_t *__restrict__ err, const uint32_t *__restrict__ order) {
   __shared__ uint2 s_stk[32][kWideStack];
   __shared__ WideSlot s_res[32];
   if (scene->nbranches > wide_cap) return;  // trace_node2_kernel traces the rays
@@ -1203,7 +1198,6 @@ trace_wide_kernel(const WideRec *__restrict__ wide, uint32_t wide_cap,
       const uint32_t state = !w.fail && p.defer ? (p.viol ? 3u : 1u) : 0u;
       s_res[group] = WideSlot{C.m, C.u, C.v, C.j, state};
     }
-    add_stats(stats, w, 0);
   }
   // the other warps only arrive
   if (threadIdx.x >= 32) {
@@ -1519,8 +1513,8 @@ __device__ __forceinline__ void take_tet(Best &b, double te, double e1, double e
 // away.  The reference pops a node and then tests its box; here a branch
 // tests both children's, half as many dependent loads, and a popped entry
 // compares its entry distance with the running distance, which is all of
-// that test that can have changed.  Steps count as the reference's pops: two
-// per entered branch.
+// that test that can have changed.  Steps and nodes count as the reference's
+// pops: the root, and two per entered branch.
 template <bool WINDOW, typename P = float4>
 __device__ void walkT(const NodeT *__restrict__ nodes, const P *__restrict__ prims,
                       const uint32_t *__restrict__ sidx, const CtxT &c, float bnd,
@@ -1535,6 +1529,7 @@ __device__ void walkT(const NodeT *__restrict__ nodes, const P *__restrict__ pri
     const float4 a = __ldg(np), bb = __ldg(np + 1);
     float te;
     w.it++;
+    w.branch++;
     if (ray_aabb_t<false>(WINDOW ? bnd : t, a.x, a.y, a.z, bb.x, bb.y, bb.z, c.r, te)) {
       stk[0] = make_uint2(__float_as_uint(bb.w), __float_as_uint(a.w));
       stt[0] = te;
@@ -1549,7 +1544,7 @@ __device__ void walkT(const NodeT *__restrict__ nodes, const P *__restrict__ pri
       const float et = stt[sp--];
       if (!(et <= (WINDOW ? bnd : t))) continue;
       if (e.y & kLeafBit) { lref = e.x; lcnt = e.y & kCountMask; break; }
-      w.branch++;
+      w.branch += 2;
       w.it += 2;
       const float4 *cp = reinterpret_cast<const float4 *>(nodes + e.x);
       const float4 a0 = __ldg(cp), b0 = __ldg(cp + 1), a1 = __ldg(cp + 2), b1 = __ldg(cp + 3);
@@ -1626,6 +1621,7 @@ __device__ void walkT_warp(const NodeT *__restrict__ nodes, const P *__restrict_
     const float4 a = __ldg(np), bb = __ldg(np + 1);
     float te;
     w.it++;
+    if (lane == 0) w.branch++;
     if (ray_aabb_t<false>(WINDOW ? bnd : t, a.x, a.y, a.z, bb.x, bb.y, bb.z, c.r, te)) {
       sp = 0;
       if (lane == 0)
@@ -1639,7 +1635,7 @@ __device__ void walkT_warp(const NodeT *__restrict__ nodes, const P *__restrict_
     __syncwarp();  // read by every lane before a push overwrites it
     if (!(__uint_as_float(e.z) <= (WINDOW ? bnd : t))) continue;
     if (!(e.y & kLeafBit)) {
-      if (lane == 0) w.branch++;
+      if (lane == 0) w.branch += 2;
       w.it += 2;
       const float4 *cp = reinterpret_cast<const float4 *>(nodes + e.x);
       const float4 a0 = __ldg(cp), b0 = __ldg(cp + 1), a1 = __ldg(cp + 2), b1 = __ldg(cp + 3);
@@ -2082,16 +2078,15 @@ int resident_blocks(const void *fn, int block) {
 
 // The first pass over the wide nodes.
 static void launch_wide(srt_accel *a, const srt_ray *rays, size_t n, srt_hit *hits,
-                        const float *prev_normals, float *normal_out, unsigned long long *stats,
-                        Deferred *dlist, uint32_t *dcount, uint32_t max_iter,
-                        const uint32_t *order) {
+                        const float *prev_normals, float *normal_out, Deferred *dlist,
+                        uint32_t *dcount, uint32_t max_iter, const uint32_t *order) {
   srt_ctx *ctx = a->ctx;
   const auto kern = a->kind == SRT_TRIANGLES ? trace_wide_kernel<SRT_TRIANGLES>
                                              : trace_wide_kernel<SRT_SPHERES>;
   kern<<<(unsigned)((n + 31) / 32), 128, 0, ctx->stream>>>(
       a->wide, a->wide_cap, a->nodes.as<Node2>(), a->prims.as<float4>(),
       a->indices.as<uint32_t>(), rays, n, hits, a->scene.as<SceneInfo>(), prev_normals,
-      normal_out, stats, dlist, dcount, max_iter, ctx->d_err, order);
+      normal_out, dlist, dcount, max_iter, ctx->d_err, order);
   ctx->launches++;
 }
 
@@ -2151,14 +2146,14 @@ srt_status launch_trace(srt_accel *a, const srt_ray *rays, size_t n, srt_hit *hi
       const float4 *pr = a->prims.as<float4>();
       const uint32_t *ix = a->indices.as<uint32_t>();
       const bool tri = a->kind == SRT_TRIANGLES;
-      // a caller's cap counts the two-child walk's steps, and a full-grid
-      // launch is that kernel's; a tree that may have more branches than wide
-      // nodes gets both kernels, each leaving the rays to the other by the
-      // branch count
+      // a caller's cap and counters are of the two-child walk's steps, and a
+      // full-grid launch is that kernel's; a tree that may have more branches
+      // than wide nodes gets both kernels, each leaving the rays to the other
+      // by the branch count
       const bool wide =
-          !single && !max_iter_cap && !(flags & SRT_TRACE_GRID) && takes_wide(a, n);
+          !single && !max_iter_cap && !stats && !(flags & SRT_TRACE_GRID) && takes_wide(a, n);
       if (wide)
-        launch_wide(a, rays, n, hits, pn, normal_out, stats, dlist, dcount, max_iter, order);
+        launch_wide(a, rays, n, hits, pn, normal_out, dlist, dcount, max_iter, order);
       if (!wide || !a->wide_all) {
         const auto kern = tri ? (single ? trace_node2_kernel<SRT_TRIANGLES, true>
                                         : trace_node2_kernel<SRT_TRIANGLES, false>)
@@ -3086,7 +3081,7 @@ extern "C" SRT_API srt_status srt_trace_closest_noalloc(srt_accel *a, const srt_
   switch (a->kind) {
     case SRT_TRIANGLES: {
       const Node2 *nd = a->nodes.as<Node2>();
-      launch_wide(a, rays, n, hits, nullptr, nullptr, nullptr, dlist, dcount, max_iter, nullptr);
+      launch_wide(a, rays, n, hits, nullptr, nullptr, dlist, dcount, max_iter, nullptr);
       if (!a->wide_all) {
         trace_node2_kernel<SRT_TRIANGLES, false><<<grid, block, 0, st>>>(
             nd, pr, ix, rays, n, hits, scene, nullptr, nullptr, nullptr, dlist, dcount, max_iter,
@@ -3101,7 +3096,7 @@ extern "C" SRT_API srt_status srt_trace_closest_noalloc(srt_accel *a, const srt_
     }
     case SRT_SPHERES: {
       const Node2 *nd = a->nodes.as<Node2>();
-      launch_wide(a, rays, n, hits, nullptr, nullptr, nullptr, dlist, dcount, max_iter, nullptr);
+      launch_wide(a, rays, n, hits, nullptr, nullptr, dlist, dcount, max_iter, nullptr);
       if (!a->wide_all) {
         trace_node2_kernel<SRT_SPHERES, false><<<grid, block, 0, st>>>(
             nd, pr, ix, rays, n, hits, scene, nullptr, nullptr, nullptr, dlist, dcount, max_iter,
