@@ -1580,6 +1580,7 @@ __device__ void walkT(const NodeT *__restrict__ nodes, const P *__restrict__ pri
       }
     }
   }
+  if (w.it > max_iter) w.fail = true;  // children missed at the end are popped too
 }
 
 __device__ __forceinline__ double window_hi(double m) {
@@ -1684,6 +1685,7 @@ __device__ void walkT_warp(const NodeT *__restrict__ nodes, const P *__restrict_
                  __shfl_sync(kAll, f, src), __shfl_sync(kAll, ef, src));
     }
   }
+  if (w.it > max_iter) w.fail = true;
 }
 
 // An open ray's replay: the reference's walk from the pass's bound (full) or
