@@ -666,9 +666,10 @@ SRT_API srt_status srt_batch_config(srt_batch *b, int32_t *block,
                                     uint64_t *kernels_per_call);
 /* The traversal point the autotuner picked on the batch's first call: block
  * size, grabs of 32 rays per warp, traversal stack depth (24, 32 or 48
- * entries) and ray order (0: in tiles of the scenes' rows of rays, array
- * order where there are none; 12 or 22: sorted within each scene by that many
- * top bits of a Morton code over origin and direction). */
+ * entries) and ray order (0: unsorted, that is array order or, in scenes whose
+ * rays come in rows and where it was the faster, tiles of the rows; 12 or 22:
+ * sorted within each scene by that many top bits of a Morton code over origin
+ * and direction). */
 SRT_API srt_status srt_batch_tuning(srt_batch *b, int32_t *block,
                                     int32_t *rays_per_grab, int32_t *stack_depth,
                                     int32_t *sort_bits);

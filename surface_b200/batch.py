@@ -71,8 +71,8 @@ class TriangleBatch:
 
     def tuning(self):
         """The autotuned traversal point: {"block", "rays_per_grab",
-        "stack_depth", "sort_bits"} (sort_bits 0: rays in tiles of
-        their rows, array order where there are none)."""
+        "stack_depth", "sort_bits"} (sort_bits 0: rays unsorted, in
+        array order or in tiles of their rows)."""
         v = [C.c_int32() for _ in range(4)]
         check(self.L.srt_batch_tuning(self.h, *[C.byref(x) for x in v]))
         return dict(zip(("block", "rays_per_grab", "stack_depth", "sort_bits"),

@@ -6,9 +6,9 @@
 // traversal (timed with CUDA events, one axis at a time from the default
 // point): block size x rays per grab, then the traversal stack depth (24, 32
 // or 48 entries; a depth the trees overflow is dropped), then the ray order
-// (tiles of the rays' rows, or sorted within each scene by the top 12 or 22
-// bits of a Morton code over origin and direction, the sort timed with the
-// trace).
+// (tiles of the rays' rows in the scenes whose rays come in rows, array order
+// for all, or sorted within each scene by the top 12 or 22 bits of a Morton
+// code over origin and direction, the ordering timed with the trace).
 // The second identical call captures the whole sequence in a CUDA graph,
 // later identical calls replay it with one graph launch.
 #include <cstring>
@@ -27,7 +27,8 @@ struct srt_batch {
   const srt_ray *rays = nullptr;
   srt_hit *hits = nullptr;
   int block = 128, R = 1, depth = 32, sort_bits = 0;
-  DevBuf rkey, rorder;  // batch ray order (sort_bits > 0)
+  bool tiles = true;            // unsorted rays in tiles of their rows
+  DevBuf rkey, rorder, rwidth;  // sort keys, order, row length per scene
   bool tuned = false, pinned = false;  // pinned: set by srt_batch_set_tuning
   int same_calls = 0;
   cudaGraph_t graph = nullptr;
@@ -74,17 +75,20 @@ srt_status upload_offsets(srt_batch *b) {
   return SRT_OK;
 }
 
-// The traversal as tuned: the batch ray order (when sorting) and the trace.
-srt_status trace_tuned(srt_batch *b, int block, int R, int depth, int sort_bits) {
+// The traversal as tuned: the ray order and the trace.
+srt_status trace_tuned(srt_batch *b, int block, int R, int depth, int sort_bits, bool tiles) {
   const size_t n = b->bt.nrays;
   cudaError_t e;
-  if (sort_bits == 0) {  // the scenes' rays in tiles of their rows
-    if (b->rorder.ensure(n * 4) != cudaSuccess)  // array order does as well
+  const uint32_t *width = nullptr;
+  if (sort_bits == 0) {
+    if (!tiles || b->rorder.ensure(n * 4) != cudaSuccess ||  // array order does as well
+        b->rwidth.ensure((size_t)b->bt.nseg * 4) != cudaSuccess)
       return launch_trace_batch(b->ctx, b->bt, b->rays, b->hits, block, R, nullptr, depth,
                                 nullptr);
-    srt_status s = raster_order(b->ctx, b->rays, n, b->bt.roff.as<uint32_t>(), b->bt.nseg,
-                                b->rorder.as<uint32_t>());
+    srt_status s = batch_raster_order(b->ctx, b->rays, n, b->bt.roff.as<uint32_t>(), b->bt.nseg,
+                                      b->rwidth.as<uint32_t>(), b->rorder.as<uint32_t>());
     if (s != SRT_OK) return s;
+    width = b->rwidth.as<uint32_t>();
   } else {
     if ((e = b->rkey.ensure(n * 4 + 64)) != cudaSuccess ||
         (e = b->rorder.ensure(n * 4)) != cudaSuccess)
@@ -94,13 +98,13 @@ srt_status trace_tuned(srt_batch *b, int block, int R, int depth, int sort_bits)
     if (s != SRT_OK) return s;
   }
   return launch_trace_batch(b->ctx, b->bt, b->rays, b->hits, block, R, nullptr, depth,
-                            b->rorder.as<uint32_t>());
+                            b->rorder.as<uint32_t>(), width);
 }
 
 srt_status build_and_trace(srt_batch *b, const uint32_t *h_foff) {
   srt_status s = build_batch(b->ctx, b->bt, b->verts, b->faces, h_foff, b->bt.nseg);
   if (s != SRT_OK) return s;
-  return trace_tuned(b, b->block, b->R, b->depth, b->sort_bits);
+  return trace_tuned(b, b->block, b->R, b->depth, b->sort_bits, b->tiles);
 }
 
 // Reads and clears the kernels' limit word: whether a candidate's walks
@@ -123,7 +127,7 @@ srt_status autotune(srt_batch *b) {
   static const int blocks[] = {64, 128, 256};
   static const int Rs[] = {1, 2, 4};
   static const int depths[] = {24, 32, 48};
-  static const int sorts[] = {0, 12, 22};
+  static const int sorts[] = {0, 12, 22};  // (0: array order, tiles being the default)
   srt_ctx *ctx = b->ctx;
   cudaStream_t st = ctx->stream;
   bool pending = false;  // a limit raised before tuning (the build's) stays for the caller
@@ -139,12 +143,13 @@ srt_status autotune(srt_batch *b) {
   cudaEventCreate(&e1);
   // ms of one candidate (second of two runs: the first warms caches); ok
   // false when its walks overflowed the stack
-  auto time_point = [&](int blk, int r, int dep, int sb, float &ms, bool &ok) -> srt_status {
+  auto time_point = [&](int blk, int r, int dep, int sb, bool tl, float &ms,
+                        bool &ok) -> srt_status {
     ms = 0.0f;
     ok = true;
     for (int rep = 0; rep < 2; rep++) {
       cudaEventRecord(e0, st);
-      srt_status s = trace_tuned(b, blk, r, dep, sb);
+      srt_status s = trace_tuned(b, blk, r, dep, sb, tl);
       cudaEventRecord(e1, st);
       if (s != SRT_OK) return s;
       cudaError_t e = cudaEventSynchronize(e1);
@@ -160,28 +165,29 @@ srt_status autotune(srt_batch *b) {
     return SRT_OK;
   };
   int bb = 128, br = 1, bd = 32, bs = 0;
+  bool bt = true;
   float best = 1e30f;
   srt_status s = SRT_OK;
   for (int blk : blocks)
     for (int r : Rs) {
       float ms;
       bool ok;
-      if ((s = time_point(blk, r, bd, bs, ms, ok)) != SRT_OK) break;
+      if ((s = time_point(blk, r, bd, bs, bt, ms, ok)) != SRT_OK) break;
       if (ok && ms < best) best = ms, bb = blk, br = r;
     }
   for (int dep : depths) {
     if (s != SRT_OK || dep == bd || (pending && dep < 32)) continue;
     float ms;
     bool ok;
-    if ((s = time_point(bb, br, dep, bs, ms, ok)) != SRT_OK) break;
+    if ((s = time_point(bb, br, dep, bs, bt, ms, ok)) != SRT_OK) break;
     if (ok && ms < best) best = ms, bd = dep;
   }
   for (int sb : sorts) {
-    if (s != SRT_OK || sb == bs) continue;
+    if (s != SRT_OK) continue;
     float ms;
     bool ok;
-    if ((s = time_point(bb, br, bd, sb, ms, ok)) != SRT_OK) break;
-    if (ok && ms < best) best = ms, bs = sb;
+    if ((s = time_point(bb, br, bd, sb, false, ms, ok)) != SRT_OK) break;
+    if (ok && ms < best) best = ms, bs = sb, bt = false;
   }
   cudaEventDestroy(e0);
   cudaEventDestroy(e1);
@@ -190,6 +196,7 @@ srt_status autotune(srt_batch *b) {
   b->R = br;
   b->depth = bd;
   b->sort_bits = bs;
+  b->tiles = bt;
   b->tuned = true;
   return SRT_OK;
 }
@@ -251,6 +258,7 @@ SRT_API srt_status srt_batch_set_tuning(srt_batch *b, int32_t block, int32_t ray
   b->R = rays_per_grab;
   b->depth = stack_depth;
   b->sort_bits = sort_bits;
+  b->tiles = true;
   b->tuned = true;
   b->pinned = true;
   return SRT_OK;
@@ -329,7 +337,7 @@ SRT_API srt_status srt_batch_build_trace(srt_batch *b, int32_t nscenes, const fl
   const uint64_t lb = ctx->launches;
   if (!b->tuned && (s = autotune(b)) != SRT_OK) return s;
   const uint64_t lt = ctx->launches;
-  if ((s = trace_tuned(b, b->block, b->R, b->depth, b->sort_bits)) != SRT_OK) return s;
+  if ((s = trace_tuned(b, b->block, b->R, b->depth, b->sort_bits, b->tiles)) != SRT_OK) return s;
   b->kernels_per_call = (lb - l0) + (ctx->launches - lt);
   b->same_calls++;
   // capture on the second identical call (the legacy and per-thread default
