@@ -754,9 +754,8 @@ srt_status sort_pairs_seg(srt_ctx *ctx, uint32_t *keys, uint32_t *vals, size_t n
                           bool identity_vals, const uint32_t *seg, int nseg, int key_bits,
                           const uint32_t *skip = nullptr) {
   if (n == 0) return SRT_OK;
-  // (larger batches of scenes than a digit tells apart, and other keys, take
-  // the passes below)
-  if (key_bits > 20 && key_bits <= 30 && n > kLargeSort && n < (1u << 30) && nseg <= 256)
+  // (a batch has at most 256 scenes, as many as a digit tells apart)
+  if (key_bits > 20 && key_bits <= 30 && n > kLargeSort && n < (1u << 30))
     return sort_codes30_large(ctx, keys, vals, n, identity_vals, seg, nseg, skip);
   srt_status s = sort_scratch(ctx, n);
   if (s != SRT_OK) return s;
@@ -1336,7 +1335,7 @@ __global__ void widen_kernel(const Node2 *__restrict__ nodes,
 }
 
 // Scene box and Morton codes.  With `hist` (3 x 1024 words) and `tickets`,
-// also the digit histograms of sort_codes30's passes (hist_ready).
+// also the digit histograms of sort_codes30's passes.
 template <int KIND>
 srt_status launch_bbox_morton(srt_ctx *ctx, const float *v, const uint32_t *f,
                               const float *radius, float constr, size_t n,
@@ -1466,11 +1465,11 @@ srt_status build_kind(srt_accel *a, const float *v, const uint32_t *f,
     s = launch_bbox_morton<KIND>(ctx, v, f, radius, constr, n, scene, codes, nullptr, hist,
                                  tickets);
     if (s != SRT_OK) return s;
-    s = sort_codes30(ctx, codes, idx, n, true, true);
+    s = sort_codes30(ctx, codes, idx, n, true);
   } else {
     // the refit's boxes are written after the cache: their scratch holds the
     // packed spheres until then
-    static_assert(sizeof(BoxP) >= sizeof(float4), "a box's room holds a sphere");
+    static_assert(sizeof(BoxP) >= 2 * sizeof(float4), "n - 1 boxes hold n spheres");
     if (KIND == SRT_SPHERES) packed = ctx->s_ibox.as<float4>();
     s = launch_bbox_morton<KIND>(ctx, v, f, radius, constr, n, scene, codes, nullptr, nullptr,
                                  nullptr, packed);

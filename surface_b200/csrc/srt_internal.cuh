@@ -393,17 +393,17 @@ srt_status sort_pairs(srt_ctx *ctx, uint32_t *d_keys, uint32_t *d_vals,
                       size_t n, bool identity_vals, int key_bits = 32,
                       const uint32_t *skip = nullptr);
 // The same order for 30-bit keys (Morton codes) with one kernel per 10-bit
-// pass (srt_sort.cu); n < 2^30.
+// pass (srt_sort.cu), their digits counted before (sort_codes30_scratch).
 srt_status sort_codes30(srt_ctx *ctx, uint32_t *d_keys, uint32_t *d_vals, size_t n,
-                        bool identity_vals, bool hist_ready = false);
+                        bool identity_vals);
 // The same order for large arrays (8-bit passes over long tiles), then with
 // nseg > 1 (at most 256) a pass that groups it by the segment of each value,
 // seg the segments' offsets on the device; skip as for sort_pairs.
 srt_status sort_codes30_large(srt_ctx *ctx, uint32_t *d_keys, uint32_t *d_vals, size_t n,
                               bool identity_vals, const uint32_t *seg = nullptr, int nseg = 1,
                               const uint32_t *skip = nullptr);
-// Scratch of sort_codes30 for n keys: the digit histograms (3 x 1024 words, to be filled
-// before a hist_ready sort) and the three passes' tile counters (zeroed).
+// Scratch of sort_codes30 for n keys: the digit histograms (3 x 1024 words) and
+// the three passes' tile counters, to be filled and zeroed before the sort.
 srt_status sort_codes30_scratch(srt_ctx *ctx, size_t n, uint32_t **hist,
                                 unsigned long long **tickets);
 // The Karras tree of n >= 2 sorted codes and its emitted branches

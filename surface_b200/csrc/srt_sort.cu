@@ -2,21 +2,23 @@
 //
 // The order is the reference's: ascending 30-bit code, ties in input order
 // (RadixSort30OMP, render/render_prefix_tree_util.h:296-402, is a stable LSD
-// sort whose keys start as index = i).  Here: three 10-bit LSD passes, one
-// decoupled look-back kernel per pass:
+// sort whose keys start as index = i).  Both sorts here are one-sweep radix
+// sorts (Adinets and Merrill, 2022; the look-back is Merrill and Garland's,
+// 2016): one kernel per LSD pass instead of a count, a scan and a scatter.
+// sort_codes30, up to 2^18 codes, takes three passes of 10 bits; its digit
+// counts come from the build's Morton kernel.
 //
-//   os_hist_kernel   one read of the codes: the global count of every digit
-//                    of the three passes (shared-memory histograms, warp-
-//                    aggregated; zeroed by a memset before)
-//   os_pass_kernel   per pass, tiles of 256 x ROUNDS keys in tile order
-//                    (tile ids from a ticket counter, so a tile only waits on
-//                    tiles that are already running): rank every key within
-//                    its tile (warps own consecutive chunks, one ballot per
-//                    digit bit ranks lanes in order), publish the tile's digit
-//                    counts, add the counts of earlier tiles (look-back over
-//                    their published aggregates / inclusive prefixes), stage
-//                    the tile in shared memory in (digit, input) order and
-//                    write it out in runs of equal digits.
+//   os_pass_kernel   per pass, tiles of 1,024 keys in tile order (tile ids from
+//                    a ticket counter, so a tile only waits on tiles that are
+//                    already running): rank every key within its tile (warps
+//                    own consecutive chunks, one ballot per digit bit ranks
+//                    lanes in order), publish the tile's digit counts, add the
+//                    counts of earlier tiles (look-back over their published
+//                    aggregates / inclusive prefixes), stage the tile in shared
+//                    memory in (digit, input) order and write it out in runs of
+//                    equal digits.
+//
+// sort_codes30_large (below) takes longer tiles and shorter digits.
 //
 // Look-back words are 64 bits: the pass's epoch (a per-context counter, so
 // the status array is never cleared between passes) and a 32-bit value
@@ -35,6 +37,7 @@ constexpr int kOsBins = 1 << kOsBits;
 constexpr int kOsWarps = 8;
 constexpr int kOsThreads = kOsWarps * 32;
 constexpr int kOsPerThread = kOsBins / kOsThreads;  // 4 bins per thread
+constexpr int kOsRounds = 4;  // keys per thread: short tiles keep every SM busy
 constexpr uint32_t kFlagAgg = 1u << 30;
 constexpr uint32_t kFlagInc = 2u << 30;
 constexpr uint32_t kCountMask30 = (1u << 30) - 1u;
@@ -74,36 +77,6 @@ __device__ __forceinline__ uint32_t block_scan4(uint32_t x[kOsPerThread], uint32
   return total;
 }
 
-__global__ void __launch_bounds__(kOsThreads)
-os_hist_kernel(const uint32_t *__restrict__ keys, size_t n, uint32_t *__restrict__ ghist,
-               unsigned long long *__restrict__ tickets) {
-  __shared__ uint32_t h[3][kOsBins];
-  // the passes that follow on the stream take their tile ids from these
-  if (blockIdx.x == 0 && threadIdx.x < 3) tickets[threadIdx.x] = 0ull;
-  for (int i = threadIdx.x; i < 3 * kOsBins; i += kOsThreads) (&h[0][0])[i] = 0;
-  __syncthreads();
-  const int lane = threadIdx.x & 31;
-  const size_t stride = (size_t)gridDim.x * kOsThreads;
-  for (size_t base = (size_t)blockIdx.x * kOsThreads; base < n; base += stride) {
-    const size_t i = base + threadIdx.x;
-    const bool ok = i < n;
-    const uint32_t k = ok ? __ldg(&keys[i]) : 0u;
-    const unsigned act = __ballot_sync(0xffffffffu, ok);
-#pragma unroll
-    for (int p = 0; p < 3; p++) {
-      const uint32_t d = (k >> (kOsBits * p)) & (kOsBins - 1);
-      // warp-aggregated: one shared atomic per distinct digit of the warp
-      const unsigned peers = __match_any_sync(0xffffffffu, d) & act;
-      if (ok && lane == __ffs(peers) - 1) atomicAdd(&h[p][d], (uint32_t)__popc(peers));
-    }
-  }
-  __syncthreads();
-  for (int i = threadIdx.x; i < 3 * kOsBins; i += kOsThreads) {
-    const uint32_t c = (&h[0][0])[i];
-    if (c) atomicAdd(&ghist[i], c);
-  }
-}
-
 __device__ __forceinline__ unsigned long long ld_status(const unsigned long long *p) {
   unsigned long long v;
   asm volatile("ld.relaxed.gpu.global.u64 %0, [%1];" : "=l"(v) : "l"(p) : "memory");
@@ -124,9 +97,8 @@ __device__ __forceinline__ void st_word(uint32_t *p, uint32_t v) {
 
 // Shared memory of one pass block (dynamic): per-warp digit counts, then the
 // staged tile.
-template <int ROUNDS>
 struct PassSmem {
-  static constexpr int kTile = kOsThreads * ROUNDS;
+  static constexpr int kTile = kOsThreads * kOsRounds;
   uint32_t wc[kOsWarps][kOsBins];  // counts, then exclusive offsets per warp
   uint32_t tloc[kOsBins];          // tile-local start of each digit
   uint32_t gdst[kOsBins];          // global position of tile slot 0 per digit
@@ -136,7 +108,6 @@ struct PassSmem {
   uint32_t val[kTile];
 };
 
-template <int ROUNDS>
 __global__ void __launch_bounds__(kOsThreads)
 os_pass_kernel(const uint32_t *__restrict__ kin, const uint32_t *__restrict__ vin,
                uint32_t *__restrict__ kout, uint32_t *__restrict__ vout, uint32_t n, int shift,
@@ -144,8 +115,8 @@ os_pass_kernel(const uint32_t *__restrict__ kin, const uint32_t *__restrict__ vi
                unsigned long long *__restrict__ ticket, uint32_t epoch,
                uint32_t *__restrict__ err) {
   extern __shared__ __align__(16) unsigned char smem_raw[];
-  PassSmem<ROUNDS> &S = *reinterpret_cast<PassSmem<ROUNDS> *>(smem_raw);
-  constexpr int kTile = PassSmem<ROUNDS>::kTile;
+  PassSmem &S = *reinterpret_cast<PassSmem *>(smem_raw);
+  constexpr int ROUNDS = kOsRounds, kTile = PassSmem::kTile;
   const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
   if (threadIdx.x == 0) S.tile = (uint32_t)atomicAdd(ticket, 1ull);
   for (int i = threadIdx.x; i < kOsWarps * kOsBins; i += kOsThreads) (&S.wc[0][0])[i] = 0;
@@ -315,48 +286,6 @@ os_pass_kernel(const uint32_t *__restrict__ kin, const uint32_t *__restrict__ vi
   }
 }
 
-template <int ROUNDS>
-srt_status os_sort(srt_ctx *ctx, uint32_t *keys, uint32_t *vals, size_t n, bool identity_vals,
-                   bool hist_ready) {
-  cudaStream_t st = ctx->stream;
-  constexpr int kTile = PassSmem<ROUNDS>::kTile;
-  const uint32_t ntiles = (uint32_t)((n + kTile - 1) / kTile);
-  const size_t smem = sizeof(PassSmem<ROUNDS>);
-  static bool attr_set[64] = {};
-  if (ctx->device >= 0 && ctx->device < 64 && !attr_set[ctx->device]) {
-    cudaError_t e = cudaFuncSetAttribute(os_pass_kernel<ROUNDS>,
-                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
-                                         (int)smem);
-    if (e != cudaSuccess) return cuda_status(e, "sort pass attributes");
-    attr_set[ctx->device] = true;
-  }
-  uint32_t *ghist = nullptr;
-  unsigned long long *tickets = nullptr;
-  srt_status s = sort_codes30_scratch(ctx, n, &ghist, &tickets);
-  if (s != SRT_OK) return s;
-  unsigned long long *status = tickets + 32;  // after the 256-byte header
-  if (!hist_ready) {
-    cudaError_t e = cudaMemsetAsync(ghist, 0, 3 * kOsBins * 4, st);
-    if (e != cudaSuccess) return cuda_status(e, "sort");
-    // each block flushes up to 3 x 1024 counters: about 4096 keys per block
-    const int hgrid = (int)std::min<size_t>((n + 4095) / 4096, (size_t)ctx->num_sms * 2);
-    os_hist_kernel<<<hgrid, kOsThreads, 0, st>>>(keys, n, ghist, tickets);
-    ctx->launches++;
-  }
-  // keys -> 2 -> 3 -> keys: three passes end where they started
-  uint32_t *ksrc[3] = {keys, ctx->s_keys2.as<uint32_t>(), ctx->s_keys3.as<uint32_t>()};
-  uint32_t *vsrc[3] = {vals, ctx->s_vals2.as<uint32_t>(), ctx->s_vals3.as<uint32_t>()};
-  for (int p = 0; p < 3; p++) {
-    const uint32_t epoch = ++ctx->os_epoch == 0 ? ++ctx->os_epoch : ctx->os_epoch;
-    const uint32_t *vin = (p == 0 && identity_vals) ? nullptr : vsrc[p];
-    os_pass_kernel<ROUNDS><<<ntiles, kOsThreads, smem, st>>>(
-        ksrc[p], vin, ksrc[(p + 1) % 3], vsrc[(p + 1) % 3], (uint32_t)n, kOsBits * p,
-        ghist + kOsBins * p, status, tickets + p, epoch, ctx->d_err);
-    ctx->launches++;
-  }
-  return cuda_status(cudaGetLastError(), "sort passes");
-}
-
 // ------------------------------------------------------------ large arrays
 // What counts above some 10^5 keys is how the keys leave a pass: a tile of
 // 4,096 keys in 1,024 digits writes runs of 4 keys, half of every 32-byte
@@ -376,7 +305,7 @@ constexpr int kLgWarps = 16;
 constexpr int kLgThreads = kLgWarps * 32;
 constexpr int kLgRounds = 16;
 constexpr int kLgTile = kLgThreads * kLgRounds;
-constexpr int kLgPasses = 4;  // digits of 8, 8, 7 and 7 bits: 30
+constexpr int kLgPasses = 4;  // digits of 8, 8, 8 and 6 bits: 30
 
 // Counts of every digit of the passes.
 __global__ void __launch_bounds__(kLgThreads)
@@ -628,8 +557,8 @@ srt_status sort_codes30_large(srt_ctx *ctx, uint32_t *keys, uint32_t *vals, size
     const uint32_t *vin = (p == 0 && identity_vals) ? nullptr : vb[way[p]];
     const auto kern = p < kLgPasses ? lg_pass_kernel<false> : lg_pass_kernel<true>;
     kern<<<ntiles, kLgThreads, sizeof(LgSmem), st>>>(
-        kb[way[p]], vin, kb[way[p + 1]], vb[way[p + 1]], (uint32_t)n, kLgBits * p,
-        ghist + kLgBins * p, seg, nseg, status + (size_t)p * ntiles * kLgBins, tickets + p,
+        kb[way[p]], vin, kb[way[p + 1]], vb[way[p + 1]], (uint32_t)n,
+        p < kLgPasses ? kLgBits * p : 0, ghist + kLgBins * (p % kLgPasses), seg, nseg, status + (size_t)p * ntiles * kLgBins, tickets + p,
         ctx->d_err, skip);
     ctx->launches++;
   }
@@ -662,20 +591,43 @@ srt_status sort_codes30_scratch(srt_ctx *ctx, size_t n, uint32_t **hist,
 }
 
 // Stable sort of (30-bit code, value) pairs by code, in place.  identity_vals:
-// the values are 0..n-1 on entry (not read).  hist_ready: the digit
-// histograms of the three passes are already in the scratch and the tile
-// counters zeroed (the Morton kernel of a build does both).  n < 2^30.
+// the values are 0..n-1 on entry (not read).  The digit histograms of the three
+// passes are already in the scratch and the tile counters zeroed (the Morton
+// kernel of a build does both).
 srt_status sort_codes30(srt_ctx *ctx, uint32_t *keys, uint32_t *vals, size_t n,
-                        bool identity_vals, bool hist_ready) {
+                        bool identity_vals) {
   if (n == 0) return SRT_OK;
   if (n >= (1u << 30)) {
     set_error("sort: at most 2^30 - 1 keys");
     return SRT_ERR_INVALID;
   }
-  // small arrays: short tiles keep every SM busy; large: long tiles amortise
-  // the per-tile look-back
-  if (n <= (1u << 21)) return os_sort<4>(ctx, keys, vals, n, identity_vals, hist_ready);
-  return os_sort<16>(ctx, keys, vals, n, identity_vals, hist_ready);
+  const uint32_t ntiles = (uint32_t)((n + PassSmem::kTile - 1) / PassSmem::kTile);
+  const size_t smem = sizeof(PassSmem);
+  static bool attr_set[64] = {};
+  if (ctx->device >= 0 && ctx->device < 64 && !attr_set[ctx->device]) {
+    cudaError_t e = cudaFuncSetAttribute(os_pass_kernel,
+                                         cudaFuncAttributeMaxDynamicSharedMemorySize,
+                                         (int)smem);
+    if (e != cudaSuccess) return cuda_status(e, "sort pass attributes");
+    attr_set[ctx->device] = true;
+  }
+  uint32_t *ghist = nullptr;
+  unsigned long long *tickets = nullptr;
+  srt_status s = sort_codes30_scratch(ctx, n, &ghist, &tickets);
+  if (s != SRT_OK) return s;
+  unsigned long long *status = tickets + 32;  // after the 256-byte header
+  // keys -> 2 -> 3 -> keys: three passes end where they started
+  uint32_t *ksrc[3] = {keys, ctx->s_keys2.as<uint32_t>(), ctx->s_keys3.as<uint32_t>()};
+  uint32_t *vsrc[3] = {vals, ctx->s_vals2.as<uint32_t>(), ctx->s_vals3.as<uint32_t>()};
+  for (int p = 0; p < 3; p++) {
+    const uint32_t epoch = ++ctx->os_epoch == 0 ? ++ctx->os_epoch : ctx->os_epoch;
+    const uint32_t *vin = (p == 0 && identity_vals) ? nullptr : vsrc[p];
+    os_pass_kernel<<<ntiles, kOsThreads, smem, ctx->stream>>>(
+        ksrc[p], vin, ksrc[(p + 1) % 3], vsrc[(p + 1) % 3], (uint32_t)n, kOsBits * p,
+        ghist + kOsBins * p, status, tickets + p, epoch, ctx->d_err);
+    ctx->launches++;
+  }
+  return cuda_status(cudaGetLastError(), "sort passes");
 }
 
 }  // namespace srt
