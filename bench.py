@@ -23,7 +23,9 @@ rays copied in, hits and scalars copied out every step).
 
 ``--impl reference`` times the reference's own CPU code (Build32 + OpenMP
 Traverse, compiled from its sources into oracle/_ref) on the host cores, for
-every ray of the step (nothing sampled or scaled).
+every ray of the step (nothing sampled or scaled); where that is not built it
+prints an "unavailable" line, for texture, lines and solids the time of the
+restatement, named as such.
 """
 from __future__ import annotations
 
@@ -174,6 +176,13 @@ PROFILES = os.path.join(ROOT, "profiles")
 TRAFFIC_PROFILE = {"tet": "trace_tet_kernel.tet64.md"}
 
 
+# the walks' and marches' rooflines: achieved and frac are of bytes that the
+# caches serve, not of DRAM traffic
+CACHED = ("algorithmic bytes (visits counted on the two-child walk) over time; L1 and L2 serve "
+          "them, so frac is no share of the HBM rate: profiles/counters.md has DRAM bytes and "
+          "issue slots")
+
+
 def profiled_traffic(kind):
     try:
         with open(os.path.join(PROFILES, TRAFFIC_PROFILE[kind])) as f:
@@ -186,7 +195,7 @@ def profiled_traffic(kind):
 
 
 def algorithmic_bytes_per_ray(kind, stats, nrays):
-    """Per-ray bytes the traversal must move: ray (32) + hit (16) + nodes
+    """Per-ray bytes the two-child walk must move: ray (32) + hit (16) + nodes
     visited x node size + primitives tested x primitive record."""
     branch, leaf, prim = (float(x) / nrays for x in stats)
     if kind == "tet":
@@ -548,6 +557,13 @@ def run_reference_arm(args, W):
     if rank != 0:
         return
     cores = os.cpu_count() or 1
+    from oracle import oracle as O
+    if W["kind"] in ("tri", "tet", "sphere", "batched", "frame") and not O.have_ref():
+        print(json.dumps({"impl": "reference", "unavailable":
+                          "the reference's own CPU code is not built here (its sources are "
+                          "absent, so oracle/_ref is); this repository's restatement of it "
+                          "is no reference"}), flush=True)
+        return
     step = {"batched": cpu_reference_batched, "sphere": cpu_reference_particles,
             "frame": cpu_reference_frame, "scene": cpu_reference_scene,
             "texture": cpu_reference_texture, "lines": cpu_reference_lines,
@@ -596,6 +612,10 @@ def run_reference_arm(args, W):
         sample = (f"every fetch ({ns}) per step through the reference's own "
                   f"SparseVolumeAccel (Build + Sample) over {cores} threads; median of "
                   f"{args.steps}")
+    if kind == "port" and W["kind"] in ("texture", "lines", "solids"):
+        sample = (f"{ns} fetches or rays of a full step through this repository's restatement "
+                  f"of the reference's CPU code (the reference's own is not built here), "
+                  f"{cores} threads; median of {args.steps}")
     line = {
         "impl": "reference",
         "metric": {"batched": METRIC_BATCH, "sphere": METRIC_PART,
@@ -752,7 +772,7 @@ def run_volume(args, W):
     nsamp = volume_sample_count(p)
     bwd_ms = fb_ms - f_ms
     uniq = 2 * W["dens"].nbytes + nr * (16 + 4 + 16) + 2 * W["tf"].nbytes
-    roofline = {"bound": "hbm", "kernel": "vol_bwd_kernel (fwd+bwd minus fwd)",
+    roofline = {"bound": "issue", "note": CACHED, "kernel": "vol_bwd_kernel (fwd+bwd minus fwd)",
                 "achieved": round(uniq / (bwd_ms * 1e-3) / 1e9, 1), "peak": hbm,
                 "unit": "GB/s", "frac": round(uniq / (bwd_ms * 1e-3) / 1e9 / hbm, 4),
                 "peak_source": src, "traffic": None,
@@ -870,7 +890,7 @@ def run_texture(args, W):
     if os.path.exists(prof):
         m = re.search(r"traffic_per_launch_bytes:\s*(\d+)", open(prof).read())
         traffic = int(m.group(1)) if m else None
-    roofline = {"bound": "hbm", "kernel": "sparse_fetch_kernel",
+    roofline = {"bound": "l1", "kernel": "sparse_fetch_kernel",
                 "achieved": round(alg / (ms * 1e-3) / 1e9, 1), "peak": hbm, "unit": "GB/s",
                 "frac": round(alg / (ms * 1e-3) / 1e9 / hbm, 4), "peak_source": src,
                 "traffic": traffic, "algorithmic_bytes_per_launch": int(alg)}
@@ -1009,7 +1029,7 @@ def run_lines(args, W):
     if os.path.exists(prof):
         m = re.search(r"traffic_per_launch_bytes:\s*(\d+)", open(prof).read())
         traffic = int(m.group(1)) if m else None
-    roofline = {"bound": "hbm", "kernel": "line_trace_kernel",
+    roofline = {"bound": "issue", "note": CACHED, "kernel": "line_trace_kernel",
                 "achieved": round(alg / (ms * 1e-3) / 1e9, 1), "peak": hbm, "unit": "GB/s",
                 "frac": round(alg / (ms * 1e-3) / 1e9 / hbm, 4), "peak_source": src,
                 "traffic": traffic, "algorithmic_bytes_per_launch": int(alg),
@@ -1136,7 +1156,7 @@ def run_solids(args, W):
     hbm, src = peaks()
     nn = acc.info()[1]
     alg = n * (32 + 40) + 112 * W["prims"].shape[0] + 32 * nn
-    roofline = {"bound": "hbm", "kernel": "solid_trace_kernel<8>",
+    roofline = {"bound": "fp64 latency", "note": CACHED, "kernel": "solid_trace_kernel<8>",
                 "achieved": round(alg / (tms * 1e-3) / 1e9, 1), "peak": hbm, "unit": "GB/s",
                 "frac": round(alg / (tms * 1e-3) / 1e9 / hbm, 4), "peak_source": src,
                 "traffic": None, "algorithmic_bytes_per_launch": int(alg),
@@ -1315,7 +1335,7 @@ def run_batched(args, W):
     trace_bytes = algorithmic_bytes_per_ray("tri", stats, nr) * nr
     build_bytes = nprim * BUILD_BYTES_PER_TRI
     achieved = (trace_bytes + build_bytes) / (ms_per_step * 1e-3) / 1e9
-    roofline = {"bound": "hbm", "kernel": "whole batched step (graph)",
+    roofline = {"bound": "issue", "note": CACHED, "kernel": "whole batched step (graph)",
                 "achieved": round(achieved, 1), "peak": hbm, "unit": "GB/s",
                 "frac": round(achieved / hbm, 4), "peak_source": src, "traffic": None,
                 "algorithmic_bytes_per_step": int(trace_bytes + build_bytes),
@@ -1496,7 +1516,8 @@ def run_particles(args, W):
     bpr = algorithmic_bytes_per_ray("sphere", stats, nr)
     pr_ms = statistics.mean(p_ms)
     achieved = bpr * nr / (pr_ms * 1e-3) / 1e9
-    roofline = {"bound": "hbm", "kernel": "primary trace", "achieved": round(achieved, 1),
+    roofline = {"bound": "issue", "note": CACHED, "kernel": "primary trace",
+                "achieved": round(achieved, 1),
                 "peak": hbm, "unit": "GB/s", "frac": round(achieved / hbm, 4),
                 "peak_source": src, "traffic": None,
                 "algorithmic_bytes_per_ray": round(bpr, 1),
@@ -1638,7 +1659,8 @@ def run_frame(args, W):
     bpr = algorithmic_bytes_per_ray("tri", stats, nr)
     tr_ms = statistics.mean(t_ms)
     achieved = bpr * nr / (tr_ms * 1e-3) / 1e9
-    roofline = {"bound": "hbm", "kernel": "trace", "achieved": round(achieved, 1),
+    roofline = {"bound": "issue", "note": CACHED, "kernel": "trace",
+                "achieved": round(achieved, 1),
                 "peak": hbm, "unit": "GB/s", "frac": round(achieved / hbm, 4),
                 "peak_source": src, "traffic": None,
                 "algorithmic_bytes_per_ray": round(bpr, 1),
@@ -1650,7 +1672,8 @@ def run_frame(args, W):
         cpu = {"value": round(cv, 4), "unit": "Mrays/s", "cores": os.cpu_count(), "kind": ck,
                "rays_write_s": round(ctr, 4), "trace_s": round(ctt, 4),
                "sample": f"every pixel ({cns} rays), median of 3: eye rays and write of "
-                         f"the CPU restatement, Traverse of the reference"}
+                         f"the CPU restatement, Traverse of the "
+                         f"{'reference' if ck == 'reference' else 'restatement'}"}
     L.srt_accel_destroy(acc)
     if rank == 0:
         line = {
@@ -1803,7 +1826,8 @@ def run_scene(args, W):
     bpr = 32 + 16 + 4 + 72 * ntop + 424 * nwalk + 64 * br + 48 * pr
     tr_ms = statistics.mean(parts[2])
     achieved = bpr * nr / (tr_ms * 1e-3) / 1e9
-    roofline = {"bound": "hbm", "kernel": "srt_scene_trace (top, walk and resolve kernels)",
+    roofline = {"bound": "issue", "note": CACHED,
+                "kernel": "srt_scene_trace (top, walk and resolve kernels)",
                 "achieved": round(achieved, 1),
                 "peak": hbm, "unit": "GB/s", "frac": round(achieved / hbm, 4),
                 "peak_source": src, "traffic": None,
@@ -1986,7 +2010,8 @@ def run_ours(args, W):
     bpr = algorithmic_bytes_per_ray(kind, stats, nr)
     tr_ms = statistics.mean(trace_ms)
     achieved = bpr * nr / (tr_ms * 1e-3) / 1e9
-    roofline = {"bound": "hbm", "kernel": "trace", "achieved": round(achieved, 1),
+    roofline = {"bound": "issue", "note": CACHED, "kernel": "trace",
+                "achieved": round(achieved, 1),
                 "peak": hbm, "unit": "GB/s", "frac": round(achieved / hbm, 4),
                 "peak_source": src, "traffic": profiled_traffic(kind),
                 "traffic_source": (f"profiles/{TRAFFIC_PROFILE[kind]} (first-pass kernel)"
