@@ -749,7 +749,7 @@ struct SharedStack {
   __shared__ float NAME##_t[kShDepth][NT];                 \
   SharedStack<NT> NAME(NAME##_e, NAME##_t)
 
-// A component the slab test's products can turn into NaN.
+// A component the slab test's products can turn into NaN or the wrong way round.
 __device__ __forceinline__ bool odd_ray(const RayF &r) {
   bool odd = false;
 #pragma unroll
@@ -757,8 +757,30 @@ __device__ __forceinline__ bool odd_ray(const RayF &r) {
     odd = odd || !(fabsf(r.o[k]) <= FLT_MAX) || !(fabsf(r.inv[k]) <= FLT_MAX) || r.inv[k] == 0.0f;
   return odd;
 }
+// Which: bit k for a reciprocal that is infinite to the direction's own side (a component
+// of +0, as in axis-parallel views: NaN only for a box with a plane through the
+// origin), kOddRay for all else (-0, infinite and NaN components).
+constexpr uint32_t kOddRay = 8u;
+__device__ __forceinline__ uint32_t odd_parts(const RayF &r) {
+  uint32_t odd = 0;
+#pragma unroll
+  for (int k = 0; k < 3; k++) {
+    if (!(fabsf(r.o[k]) <= FLT_MAX) || r.inv[k] != r.inv[k] || r.inv[k] == 0.0f) odd |= kOddRay;
+    if (fabsf(r.inv[k]) > FLT_MAX) odd |= (r.inv[k] < 0.0f) == (r.sgn[k] != 0) ? 1u << k : kOddRay;
+  }
+  return odd;
+}
+// Whether a box needs the reference's comparisons for a ray with these bits.
+// (In the two-child walk every box of an odd ray takes them: the look at the
+// planes costs it registers and 4 % on the rays that are not odd.)
+__device__ __forceinline__ bool odd_box(uint32_t odd, const RayF &r, float lx, float ly, float lz,
+                                        float hx, float hy, float hz) {
+  return (odd & kOddRay) || ((odd & 1u) && (lx == r.o[0] || hx == r.o[0])) ||
+         ((odd & 2u) && (ly == r.o[1] || hy == r.o[1])) ||
+         ((odd & 4u) && (lz == r.o[2] || hz == r.o[2]));
+}
 
-// The slab test of boxes that are ordered (lo <= hi) by a ray that is not
+// The slab test of boxes that are ordered (lo <= hi) and, for this ray, not
 // odd: no product is NaN and the smaller of a slab's two distances is the
 // entry whatever the direction's sign, so minima and maxima give what the
 // reference's selections give, and its subtractions and products go in
@@ -914,8 +936,9 @@ __device__ __forceinline__ void pass1_node2(const Node2 *__restrict__ nodes,
 // A leaf is entered exactly when pass1_node2 enters it for the same bound:
 // the boxes of regular trees nest and the slab arithmetic is monotone, so a
 // ray that enters a grandchild's box enters the child's no later.  Where that
-// does not hold (a zero, infinite or NaN ray component, whose products can be
-// NaN; boxes that do not nest) the child's box is tested too, with the
+// does not hold (odd rays and boxes: an axis-parallel ray that enters a
+// grandchild without a plane through its origin starts between the child's
+// planes too; boxes that do not nest) the child's box is tested too, with the
 // reference's comparisons.
 constexpr int kGrp = 4;
 // Entries of a group's stack, (node or leaf record, box entry distance): a
@@ -997,7 +1020,7 @@ __device__ __forceinline__ WidePass pass1_wide(const WideTree<KIND> &T, const Gr
                                                uint2 *stk, Cand &C, Work &w,
                                                uint32_t max_iter) {
   constexpr unsigned kAll = 0xffffffffu;
-  const bool odd = T.irregular || odd_ray(c.r);
+  const uint32_t odd = T.irregular ? kOddRay : odd_parts(c.r);
   const float2 nox = make_float2(-c.r.o[0], -c.r.o[0]), noy = make_float2(-c.r.o[1], -c.r.o[1]),
                noz = make_float2(-c.r.o[2], -c.r.o[2]);
   const float2 ivx = make_float2(c.r.inv[0], c.r.inv[0]), ivy = make_float2(c.r.inv[1], c.r.inv[1]),
@@ -1037,7 +1060,8 @@ __device__ __forceinline__ WidePass pass1_wide(const WideTree<KIND> &T, const Gr
       float tmin = fmaxf(fmaxf(fminf(x.x, x.y), fminf(y.x, y.y)), fminf(z.x, z.y));
       const float tmax = fminf(fminf(fmaxf(x.x, x.y), fmaxf(y.x, y.y)), fmaxf(z.x, z.y));
       bool hit = tmax > 0.0f && tmin <= fminf(tmax, bnd) && count != kNone;
-      if (odd && visit && count != kNone) {
+      if (odd && visit && count != kNone &&
+          odd_box(odd, c.r, A.x, A.z, B.x, A.y, A.w, B.y)) {
         hit = ray_aabb_t<true>(bnd, A.x, A.z, B.x, A.y, A.w, B.y, c.r, tmin);
         const float4 *np = reinterpret_cast<const float4 *>(T.nodes + e.x);
         const float4 a = __ldg(np), bb = __ldg(np + 1), cc = __ldg(np + 2);
@@ -1154,7 +1178,10 @@ struct WideSlot {
 // within diverged groups (sub-warp masks, 511 us on the second), four rounds
 // of 8 rays per warp (935 us: the longest rays end the launch), pushing all
 // but the nearest child unsorted (500 us), 8 to 12 blocks per SM by launch
-// bounds (482 to 520 us: spills).
+// bounds (482 to 520 us: spills).  Axis-parallel rays, of which every box once
+// took the reference's comparisons and its parent's as well (odd_box), 131,072
+// triangles, 1400^2 rays: 687 -> 588 us (two-child walk 595); 100,000 spheres,
+// 512^2: 252 -> 204.
 template <int KIND>
 __global__ void __launch_bounds__(128)
 trace_wide_kernel(const WideRec *__restrict__ wide, uint32_t wide_cap,
