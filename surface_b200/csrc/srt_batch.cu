@@ -79,7 +79,6 @@ srt_status upload_offsets(srt_batch *b) {
 srt_status trace_tuned(srt_batch *b, int block, int R, int depth, int sort_bits, bool tiles) {
   const size_t n = b->bt.nrays;
   cudaError_t e;
-  const uint32_t *width = nullptr;
   if (sort_bits == 0) {
     if (!tiles || b->rorder.ensure(n * 4) != cudaSuccess ||  // array order does as well
         b->rwidth.ensure((size_t)b->bt.nseg * 4) != cudaSuccess)
@@ -88,7 +87,6 @@ srt_status trace_tuned(srt_batch *b, int block, int R, int depth, int sort_bits,
     srt_status s = batch_raster_order(b->ctx, b->rays, n, b->bt.roff.as<uint32_t>(), b->bt.nseg,
                                       b->rwidth.as<uint32_t>(), b->rorder.as<uint32_t>());
     if (s != SRT_OK) return s;
-    width = b->rwidth.as<uint32_t>();
   } else {
     if ((e = b->rkey.ensure(n * 4 + 64)) != cudaSuccess ||
         (e = b->rorder.ensure(n * 4)) != cudaSuccess)
@@ -98,7 +96,7 @@ srt_status trace_tuned(srt_batch *b, int block, int R, int depth, int sort_bits,
     if (s != SRT_OK) return s;
   }
   return launch_trace_batch(b->ctx, b->bt, b->rays, b->hits, block, R, nullptr, depth,
-                            b->rorder.as<uint32_t>(), width);
+                            b->rorder.as<uint32_t>());
 }
 
 srt_status build_and_trace(srt_batch *b, const uint32_t *h_foff) {

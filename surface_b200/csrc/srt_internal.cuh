@@ -363,8 +363,7 @@ srt_status launch_scene_trace(srt_ctx *ctx, const TopNode *top, SceneWork W, uin
 // scratch, valid until the context's next order.
 srt_status raster_order(srt_ctx *ctx, const srt_ray *rays, size_t n, const uint32_t **order);
 // The same for the rays of a batch (ray offsets roff over nseg scenes, on the
-// device), scene by scene: width[s] is the length of scene s's rows, and order
-// holds its rays' tiles unless that is 0.
+// device), scene by scene; width: scratch, a word per scene.
 srt_status batch_raster_order(srt_ctx *ctx, const srt_ray *rays, size_t n, const uint32_t *roff,
                               int nseg, uint32_t *width, uint32_t *order);
 // Coherent traversal order of n rays (srt_raysort.cu), by tiles of rows or a
@@ -429,13 +428,12 @@ srt_status stage_karras(srt_ctx *ctx, const uint32_t *d_codes, size_t n,
                         uint32_t *d_child, uint8_t *d_flags);
 srt_status build_batch(srt_ctx *ctx, BatchTree &bt, const float *v, const uint32_t *f,
                        const uint32_t *h_foff, int nseg);
-// stack_depth: 24, 32 or 48 entries; order: NULL, a batch_ray_order or, with
-// its row lengths, a batch_raster_order.
+// stack_depth: 24, 32 or 48 entries; order: NULL, a batch_ray_order or a
+// batch_raster_order.
 srt_status launch_trace_batch(srt_ctx *ctx, BatchTree &bt, const srt_ray *rays,
                               srt_hit *hits, int block, int rays_per_thread,
                               unsigned long long *stats, int stack_depth = 32,
-                              const uint32_t *order = nullptr,
-                              const uint32_t *width = nullptr);
+                              const uint32_t *order = nullptr);
 
 // traversal (srt_trace.cu); max_iter 0 = the default walk cap
 srt_status launch_trace(srt_accel *a, const srt_ray *d_rays, size_t n,

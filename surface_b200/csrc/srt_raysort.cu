@@ -228,15 +228,16 @@ __device__ __forceinline__ uint32_t raster_ray(uint32_t k, uint32_t n, uint32_t 
   return h * w + (k - bh * w);
 }
 
-// order[k] for rays in rows; the array order otherwise, or (keep) left as it
-// is.  Four places per thread: their segment is looked up once.
+// order[k] for rays in rows; the array order otherwise, or (ordered) left as
+// it is.  Four places per thread: their segment is looked up once.
 __global__ void raster_fill_kernel(size_t n, const uint32_t *__restrict__ roff, int nseg,
                                    const uint32_t *__restrict__ width,
-                                   uint32_t *__restrict__ order, bool keep) {
+                                   uint32_t *__restrict__ order, bool ordered) {
   for (size_t g0 = (blockIdx.x * (size_t)blockDim.x + threadIdx.x) * 4; g0 < n;
        g0 += (size_t)gridDim.x * blockDim.x * 4) {
-    uint32_t sg = 0, first = 0, end = (uint32_t)n, w = 0, rows = 0, o[4];
+    uint32_t sg = 0, first = 0, end = (uint32_t)n, w = 0, o[4];
     if (!roff) w = __ldg(width);
+    if (ordered && !w) return;
 #pragma unroll
     for (int q = 0; q < 4; q++) {
       const uint32_t g = (uint32_t)g0 + q;
@@ -246,10 +247,8 @@ __global__ void raster_fill_kernel(size_t n, const uint32_t *__restrict__ roff, 
         end = __ldg(&roff[sg + 1]);
         w = __ldg(&width[sg]);
       }
-      rows |= w;
       o[q] = w && g < n ? first + raster_ray(g - first, end - first, w) : g;
     }
-    if (keep && !rows) continue;
     if (g0 + 4 <= n) {
       *reinterpret_cast<uint4 *>(order + g0) = make_uint4(o[0], o[1], o[2], o[3]);
     } else {
@@ -261,11 +260,11 @@ __global__ void raster_fill_kernel(size_t n, const uint32_t *__restrict__ roff, 
 }  // namespace
 
 static srt_status find_rows(srt_ctx *ctx, const srt_ray *rays, size_t n, const uint32_t *roff,
-                            int nseg, uint32_t *width, uint32_t *order, bool keep) {
+                            int nseg, uint32_t *width, uint32_t *order) {
   if (n == 0) return SRT_OK;
   raster_probe_kernel<<<(unsigned)nseg, kProbeThreads, 0, ctx->stream>>>(rays, n, roff, width);
   const unsigned grid = (unsigned)std::min<size_t>((n + 1023) / 1024, (size_t)ctx->num_sms * 8);
-  raster_fill_kernel<<<grid, 256, 0, ctx->stream>>>(n, roff, nseg, width, order, keep);
+  raster_fill_kernel<<<grid, 256, 0, ctx->stream>>>(n, roff, nseg, width, order, false);
   ctx->launches += 2;
   return cuda_status(cudaGetLastError(), "ray rows");
 }
@@ -277,12 +276,12 @@ srt_status raster_order(srt_ctx *ctx, const srt_ray *rays, size_t n, const uint3
     return SRT_OK;  // array order does as well
   *order = ctx->s_rorder.as<uint32_t>();
   return find_rows(ctx, rays, n, nullptr, 1, ctx->s_raster.as<uint32_t>(),
-                   ctx->s_rorder.as<uint32_t>(), false);
+                   ctx->s_rorder.as<uint32_t>());
 }
 
 srt_status batch_raster_order(srt_ctx *ctx, const srt_ray *rays, size_t n, const uint32_t *roff,
                               int nseg, uint32_t *width, uint32_t *order) {
-  return find_rows(ctx, rays, n, roff, nseg, width, order, true);
+  return find_rows(ctx, rays, n, roff, nseg, width, order);
 }
 
 srt_status batch_ray_order(srt_ctx *ctx, const srt_ray *rays, size_t n, const uint32_t *roff,

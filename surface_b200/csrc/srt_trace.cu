@@ -1994,8 +1994,7 @@ resolve_tet_kernel(const NodeT *__restrict__ nodes, const P *__restrict__ prims,
 // different cost balance across the GPU), finds the ray's scene from the
 // ray offsets and walks that scene's tree from its root, with a stack of
 // DEPTH entries (a walk that would need more stops with the limit error).
-// order (or NULL): the rays in a coherent order, grouped by scene; width (or
-// NULL): per scene, 0 where its rays are taken in array order all the same.
+// order (or NULL): the rays in a coherent order, grouped by scene.
 template <int DEPTH>
 __global__ void __launch_bounds__(256)
 trace_batch_kernel(const Node2 *__restrict__ nodes, const float4 *__restrict__ prims,
@@ -2005,7 +2004,7 @@ trace_batch_kernel(const Node2 *__restrict__ nodes, const float4 *__restrict__ p
                    uint32_t *__restrict__ work, int R, unsigned long long *__restrict__ stats,
                    Deferred *__restrict__ dlist, uint32_t *__restrict__ dcount,
                    uint32_t max_iter, uint32_t *__restrict__ err,
-                   const uint32_t *__restrict__ order, const uint32_t *__restrict__ width) {
+                   const uint32_t *__restrict__ order) {
   // each warp takes 32 * R rays at a time (no block-wide barrier: a warp
   // whose rays finish early takes more work at once)
   const uint32_t lane = threadIdx.x & 31u;
@@ -2017,8 +2016,8 @@ trace_batch_kernel(const Node2 *__restrict__ nodes, const float4 *__restrict__ p
     for (int r = 0; r < R; r++) {
       const uint32_t k = base + (uint32_t)r * 32u + lane;
       if (k >= total) break;
-      const int sg = seg_of(roff, nseg, k);
-      const uint32_t i = order && (!width || __ldg(&width[sg])) ? __ldg(&order[k]) : k;
+      const uint32_t i = order ? __ldg(&order[k]) : k;
+      const int sg = seg_of(roff, nseg, i);
       Ctx2 c;
       c.r = load_ray(rays, i, c.prev_prim, c.prev_t);
       c.keps = scenes[sg].keps;
@@ -2241,7 +2240,7 @@ srt_status launch_trace(srt_accel *a, const srt_ray *rays, size_t n, srt_hit *hi
 srt_status launch_trace_batch(srt_ctx *ctx, BatchTree &bt, const srt_ray *rays,
                               srt_hit *hits, int block, int R,
                               unsigned long long *stats, int depth,
-                              const uint32_t *order, const uint32_t *width) {
+                              const uint32_t *order) {
   const uint32_t total = (uint32_t)bt.nrays;
   if (total == 0) return SRT_OK;
   cudaStream_t st = ctx->stream;
@@ -2260,7 +2259,7 @@ srt_status launch_trace_batch(srt_ctx *ctx, BatchTree &bt, const srt_ray *rays,
   kern<<<ctx->num_sms * per_sm, block, 0, st>>>(
       bt.nodes.as<Node2>(), bt.prims.as<float4>(), rays, hits, bt.scenes.as<SceneInfo>(),
       bt.roots.as<uint32_t>(), bt.roff.as<uint32_t>(), bt.nseg, total, dcount + 1, R, stats,
-      dlist, dcount, max_iter, ctx->d_err, order, width);
+      dlist, dcount, max_iter, ctx->d_err, order);
   resolve_batch_kernel<<<ctx->num_sms * 8, 128, 0, st>>>(
       bt.nodes.as<Node2>(), bt.prims.as<float4>(), rays, hits, bt.scenes.as<SceneInfo>(),
       bt.roots.as<uint32_t>(), bt.roff.as<uint32_t>(), bt.nseg, stats, dlist, dcount,
