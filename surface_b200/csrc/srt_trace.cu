@@ -1252,21 +1252,28 @@ trace_wide_kernel(const WideRec *__restrict__ wide, uint32_t wide_cap,
   store_node2<KIND>(i, b, c, prims, hits, normal_out);
 }
 
-// Whether n rays take the wide walk: always below kWideRays, where one
-// thread per ray cannot fill the GPU and its longest rays (a silhouette's
-// pass 200 nodes and 600 primitives where the mean is 14 and 11) end the
-// launch; with more, only triangles in trees that are not small -- enough
-// rays hide the chains, and a two-child node costs fewer instructions per
-// ray.  Measured, wide / two-child, us:
-//   spheres       100,000: 64^2 rays 56 / 168, 512^2 205 / 247, 1024^2 572 / 536
+// Whether n rays take the wide walk: below a count at which one thread per ray
+// cannot fill the GPU and its longest rays (a silhouette's pass 200 nodes and
+// 600 primitives where the mean is 14 and 11) end the launch; with more, only
+// triangles in trees that are not small -- enough rays hide the chains, and a
+// two-child node costs fewer instructions per ray, which counts the more the
+// fewer nodes a ray visits.  Measured, wide / two-child, us (pinhole; spheres
+// and triangles of up to 40,000 gain more from the wide walk in axis-parallel
+// views):
+//   spheres     2,000: 362^2 rays 80 / 103, 512^2 119 / 109, 720^2 191 / 144
+//   spheres    15,000: 512^2 164 / 173, 600^2 189 / 194, 720^2 244 / 226
+//   spheres    40,000: 512^2 175 / 212, 720^2 277 / 263 (axis-parallel 278 / 343)
+//   spheres   100,000: 64^2 56 / 168, 512^2 193 / 280, 720^2 298 / 299, 1024^2 572 / 536
 //   spheres    12,000,000: 64^2 84 / 290, 512^2 433 / 555, 1400^2 3289 / 3247
-//   triangles       2,000: 64^2 26 / 48, 512^2 76 / 81, 1024^2 227 / 188
-//   triangles     100,000: 64^2 73 / 137, 512^2 177 / 309, 1400^2 707 / 805
+//   triangles   2,000: 64^2 26 / 48, 600^2 111 / 111, 720^2 143 / 131, 1024^2 227 / 188
+//   triangles  15,000: 600^2 142 / 161, 720^2 180 / 186
+//   triangles 100,000: 64^2 73 / 137, 512^2 155 / 263, 1400^2 707 / 805
 //   triangles   2,000,000: 64^2 118 / 215, 512^2 408 / 981, 1400^2 1217 / 1836
-constexpr size_t kWideRays = (size_t)1 << 19;
-constexpr size_t kWideTriangles = (size_t)1 << 15;
 bool takes_wide(const srt_accel *a, size_t n) {
-  return n < kWideRays || (a->kind == SRT_TRIANGLES && a->n >= kWideTriangles);
+  const bool tri = a->kind == SRT_TRIANGLES, small = a->n < ((size_t)1 << 13);
+  if (a->n >= ((size_t)1 << 15)) return tri || n < ((size_t)1 << 19);
+  if (tri) return n < (small ? (size_t)3 << 17 : (size_t)1 << 19);
+  return n < (small ? (size_t)1 << 18 : (size_t)3 << 17);
 }
 
 // Rays of a first-pass kernel: with `next` (a zeroed counter), persistent
@@ -3111,32 +3118,23 @@ extern "C" SRT_API srt_status srt_trace_closest_noalloc(srt_accel *a, const srt_
   const float4 *pr = a->prims.as<float4>();
   const uint32_t *ix = a->indices.as<uint32_t>();
   switch (a->kind) {
-    case SRT_TRIANGLES: {
-      const Node2 *nd = a->nodes.as<Node2>();
-      launch_wide(a, rays, n, hits, nullptr, nullptr, dlist, dcount, max_iter, nullptr);
-      if (!a->wide_all) {
-        trace_node2_kernel<SRT_TRIANGLES, false><<<grid, block, 0, st>>>(
-            nd, pr, ix, rays, n, hits, scene, nullptr, nullptr, nullptr, dlist, dcount, max_iter,
-            ctx->d_err, nullptr, nullptr, a->wide_cap);
-        ctx->launches++;
-      }
-      resolve_node2_kernel<SRT_TRIANGLES><<<rgrid, block, 0, st>>>(
-          nd, pr, ix, rays, hits, scene, nullptr, nullptr, nullptr, dlist, dcount, max_iter,
-          ctx->d_err);
-      break;
-    }
+    case SRT_TRIANGLES:
     case SRT_SPHERES: {
       const Node2 *nd = a->nodes.as<Node2>();
-      launch_wide(a, rays, n, hits, nullptr, nullptr, dlist, dcount, max_iter, nullptr);
-      if (!a->wide_all) {
-        trace_node2_kernel<SRT_SPHERES, false><<<grid, block, 0, st>>>(
-            nd, pr, ix, rays, n, hits, scene, nullptr, nullptr, nullptr, dlist, dcount, max_iter,
-            ctx->d_err, nullptr, nullptr, a->wide_cap);
+      const bool tri = a->kind == SRT_TRIANGLES, wide = takes_wide(a, n);
+      if (wide)
+        launch_wide(a, rays, n, hits, nullptr, nullptr, dlist, dcount, max_iter, nullptr);
+      if (!wide || !a->wide_all) {
+        const auto kern = tri ? trace_node2_kernel<SRT_TRIANGLES, false>
+                              : trace_node2_kernel<SRT_SPHERES, false>;
+        kern<<<grid, block, 0, st>>>(nd, pr, ix, rays, n, hits, scene, nullptr, nullptr, nullptr,
+                                     dlist, dcount, max_iter, ctx->d_err, nullptr, nullptr,
+                                     wide ? a->wide_cap : 0);
         ctx->launches++;
       }
-      resolve_node2_kernel<SRT_SPHERES><<<rgrid, block, 0, st>>>(
-          nd, pr, ix, rays, hits, scene, nullptr, nullptr, nullptr, dlist, dcount, max_iter,
-          ctx->d_err);
+      const auto res = tri ? resolve_node2_kernel<SRT_TRIANGLES> : resolve_node2_kernel<SRT_SPHERES>;
+      res<<<rgrid, block, 0, st>>>(nd, pr, ix, rays, hits, scene, nullptr, nullptr, nullptr, dlist,
+                                   dcount, max_iter, ctx->d_err);
       break;
     }
     case SRT_TETRAHEDRA: {
