@@ -321,7 +321,9 @@ __device__ __forceinline__ int texel_of(float u, int dim) {
 // whether the run lies in empty bricks: every step from a sample's index to
 // its texel rounds monotonically, so on an axis where both ends lie in one
 // brick the samples between them do too (PLAIN: no remap tables, no repeat
-// wrap).  Otherwise each sample looks its brick up once its texel is known.
+// wrap).  Otherwise the samples of a run look their bricks up, once their
+// texels are known, until one's is not empty (looking for every sample took
+// 13 % more time where no brick is empty, this 6 %; runs of 16 and 32: the same).
 // occ: NULL marches every sample.  256^3 blobs, 512^2 rays: 655 -> 390 us and
 // 29 us for the bricks; the same without an empty brick 650 -> 592 + 29 us;
 // 192^3, a remapped axis, 640 x 360: 433 -> 263 + 13 us.  (Jumping to each
@@ -363,6 +365,7 @@ vol_fwd_kernel(const VolConst K, const float *__restrict__ dens,
             !__ldg(&occ[(q[1][2] * nb.y + q[1][1]) * nb.x + q[1][0]]))
           continue;
       }
+      bool look = !PLAIN && occ;  // until a sample of the run lies in a brick that is not empty
       for (int s = s0; s < s1; s++) {
         const float t = t0 + ((float)s + 0.5f) * K.p.step;
         const float p[3] = {o[0] + t * d[0], o[1] + t * d[1], o[2] + t * d[2]};
@@ -373,11 +376,13 @@ vol_fwd_kernel(const VolConst K, const float *__restrict__ dens,
           u[k] = 0.5f * p[k] + 0.5f;
           if (!PLAIN) u[k] = tex_coord(K, k, u[k]);
         }
-        if (!PLAIN && occ &&
-            !__ldg(&occ[((texel_of(u[2], K.dim[2]) >> kBrickShift) * nb.y +
-                         (texel_of(u[1], K.dim[1]) >> kBrickShift)) * nb.x +
-                        (texel_of(u[0], K.dim[0]) >> kBrickShift)]))
-          continue;
+        if (look) {
+          if (!__ldg(&occ[((texel_of(u[2], K.dim[2]) >> kBrickShift) * nb.y +
+                           (texel_of(u[1], K.dim[1]) >> kBrickShift)) * nb.x +
+                          (texel_of(u[0], K.dim[0]) >> kBrickShift)]))
+            continue;
+          look = false;
+        }
         const float rho = fetch<PLAIN, EDGE>(dens, K.dim, u[0], u[1], u[2], nullptr);
         float4 c;
         int i0, i1;
