@@ -220,8 +220,9 @@ constexpr int kTableLook = 4096;  // longer tables are taken to have such values
 // thread per texel column, 81 texels each, coalesced along x; the smallest
 // and largest of a brick's nine columns through shared memory.  Bound by
 // reading the density once: 67 MB in 29 us (44 us while each row's load waited
-// for a bounds test).
-__global__ void __launch_bounds__(288)
+// for a bounds test).  TABLES: some axis has a remap table.
+template <bool TABLES>
+__global__ void __launch_bounds__(288, 4)
 vol_brick_kernel(const VolConst K, const float *__restrict__ dens, int3 nb,
                  const float4 *__restrict__ tf, uint8_t *__restrict__ occ) {
   const int3 dim = make_int3(K.dim[0], K.dim[1], K.dim[2]);
@@ -251,7 +252,7 @@ vol_brick_kernel(const VolConst K, const float *__restrict__ dens, int3 nb,
   const int last[3] = {min(first[0] + 31, nb.x - 1), by, bz}, sides[3] = {nb.x, nb.y, nb.z};
 #pragma unroll
   for (int k = 0; k < 3; k++) {
-    const int n = K.nremap[k];
+    const int n = TABLES ? K.nremap[k] : 0;
     if (!n || (first[k] > 0 && last[k] < sides[k] - 1)) continue;
     bool lo = n > kTableLook, hi = lo;
     if (!lo)
@@ -826,7 +827,9 @@ SRT_API srt_status srt_volume_march_fwd_ex(srt_ctx *ctx, const srt_volume_params
     }
   }
   if (occ) {
-    vol_brick_kernel<<<dim3((unsigned)(nb.x + 31) / 32, nb.y, nb.z), 288, 0, st>>>(
+    const auto bricks = K.nremap[0] || K.nremap[1] || K.nremap[2] ? vol_brick_kernel<true>
+                                                                  : vol_brick_kernel<false>;
+    bricks<<<dim3((unsigned)(nb.x + 31) / 32, nb.y, nb.z), 288, 0, st>>>(
         K, static_cast<const float *>(dd), nb, static_cast<const float4 *>(dt), occ);
     ctx->launches++;
   }
