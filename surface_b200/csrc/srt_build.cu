@@ -1194,6 +1194,41 @@ __device__ __forceinline__ void child_info(uint32_t c, bool kleaf,
   }
 }
 
+// One child of a two-child node; count 0: a branch.
+struct Box2 {
+  float lo[3], hi[3];
+  uint32_t ref, count;
+};
+__device__ __forceinline__ Box2 node2_child(const Node2 &n, uint32_t side) {
+  Box2 c;
+  if (side == 0) {
+    c = Box2{{n.a.x, n.a.y, n.a.z}, {n.a.w, n.b.x, n.b.y}, n.d.x, n.d.z & kCountMask};
+  } else {
+    c = Box2{{n.b.z, n.b.w, n.c.x}, {n.c.y, n.c.z, n.c.w}, n.d.y, n.d.w & kCountMask};
+  }
+  return c;
+}
+
+__device__ __forceinline__ WideRec make_wide(const Box2 &q) {
+  WideRec r;
+  r.a = make_float4(q.lo[0], q.hi[0], q.lo[1], q.hi[1]);
+  r.b = make_float4(q.lo[2], q.hi[2], __uint_as_float(q.ref), __uint_as_float(q.count));
+  return r;
+}
+__device__ __forceinline__ bool ordered_box(const float lo[3], const float hi[3]) {
+  return lo[0] <= hi[0] && lo[1] <= hi[1] && lo[2] <= hi[2];
+}
+__device__ __forceinline__ bool box_inside(const float lo[3], const float hi[3], const Box &p) {
+  bool in = true;
+#pragma unroll
+  for (int k = 0; k < 3; k++) in = in && p.lo[k] <= lo[k] && hi[k] <= p.hi[k];
+  return in;
+}
+
+// The two-child nodes and, unless there are more branches than wide_cap, the
+// wide ones: a branch's children are records of its parent, and its leaf
+// children its own.  A few microseconds, latency of the gathers; the wide nodes
+// in a kernel of their own took 3 more.
 template <int KIND>
 __global__ void emit_node2_kernel(const uint32_t *__restrict__ codes,
                                   const uint32_t *__restrict__ kchild,
@@ -1203,11 +1238,14 @@ __global__ void emit_node2_kernel(const uint32_t *__restrict__ codes,
                                   const uint32_t *__restrict__ slot,
                                   const BoxP *__restrict__ ibox,
                                   const float4 *__restrict__ prims,
-                                  const SceneInfo *__restrict__ scene,
+                                  SceneInfo *__restrict__ scene,
                                   const uint32_t *__restrict__ kidx,
-                                  Node2 *__restrict__ nodes, uint32_t *__restrict__ err) {
+                                  const uint32_t *__restrict__ kparent,
+                                  Node2 *__restrict__ nodes, WideRec *__restrict__ wide,
+                                  uint32_t wide_cap, uint32_t *__restrict__ err) {
   const float keps = scene->keps;
   const uint32_t nb = scene->nbranches;
+  if (nb > wide_cap) wide = nullptr;  // the two-child nodes are walked instead
   for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < nb;
        t += gridDim.x * blockDim.x) {
     const uint32_t i = __ldg(&kidx[t]);
@@ -1226,22 +1264,30 @@ __global__ void emit_node2_kernel(const uint32_t *__restrict__ codes,
     nd.c = make_float4(b1.lo[2], b1.hi[0], b1.hi[1], b1.hi[2]);
     nd.d = make_uint4(r0, r1, (c0 & kCountMask) | (axis << 30), c1 & kCountMask);
     nodes[t] = nd;  // slot[i] == t
+    bool regular = ordered_box(b0.lo, b0.hi) && ordered_box(b1.lo, b1.hi);
+    if (wide) {
+      const Box2 q[2] = {{{b0.lo[0], b0.lo[1], b0.lo[2]}, {b0.hi[0], b0.hi[1], b0.hi[2]}, r0, c0},
+                         {{b1.lo[0], b1.lo[1], b1.lo[2]}, {b1.hi[0], b1.hi[1], b1.hi[2]}, r1, c1}};
+#pragma unroll
+      for (int side = 0; side < 2; side++)
+        if (q[side].count) {  // a leaf: its record, and an empty one
+          Box2 none = q[side];
+          none.count = kNone;
+          wide[4 * (size_t)t + 2 * side] = make_wide(q[side]);
+          wide[4 * (size_t)t + 2 * side + 1] = make_wide(none);
+        }
+      if (i) {
+        const uint32_t p = __ldg(&kparent[i]);
+        WideRec *rec = wide + 4 * (size_t)__ldg(&slot[p]) + (kchild[p] == i ? 0 : 2);
+        rec[0] = make_wide(q[0]);
+        rec[1] = make_wide(q[1]);
+        const Box mine = box_unpack(__ldg(&ibox[i].a), __ldg(&ibox[i].b));
+        regular = regular && box_inside(q[0].lo, q[0].hi, mine) &&
+                  box_inside(q[1].lo, q[1].hi, mine);
+      }
+    }
+    if (!regular) scene->irregular = 1u;
   }
-}
-
-// One child of a two-child node; count 0: a branch.
-struct Box2 {
-  float lo[3], hi[3];
-  uint32_t ref, count;
-};
-__device__ __forceinline__ Box2 node2_child(const Node2 &n, uint32_t side) {
-  Box2 c;
-  if (side == 0) {
-    c = Box2{{n.a.x, n.a.y, n.a.z}, {n.a.w, n.b.x, n.b.y}, n.d.x, n.d.z & kCountMask};
-  } else {
-    c = Box2{{n.b.z, n.b.w, n.c.x}, {n.c.y, n.c.z, n.c.w}, n.d.y, n.d.w & kCountMask};
-  }
-  return c;
 }
 
 __device__ __forceinline__ NodeT make_tet_node(const Box &b, uint32_t meta, uint32_t ref) {
@@ -1297,10 +1343,8 @@ __global__ void emit_tet_kernel(const uint32_t *__restrict__ codes,
 }
 
 
-// The wide nodes (WideRec) of the two-child nodes, a thread per record.
-// Memory bound and small: 128 bytes written and up to 192 read per branch
-// (most of it shared by the branch's four threads), 1/12 as many branches
-// as primitives.
+// The wide nodes of a loaded tree's two-child nodes, a thread per record (a
+// built one's are emitted with them, emit_node2_kernel).
 __global__ void widen_kernel(const Node2 *__restrict__ nodes,
                              const uint32_t *__restrict__ nbranches, uint32_t cap,
                              WideRec *__restrict__ wide, uint32_t *__restrict__ irregular) {
@@ -1309,7 +1353,7 @@ __global__ void widen_kernel(const Node2 *__restrict__ nodes,
     for (uint32_t t = blockIdx.x * blockDim.x + threadIdx.x; t < 2 * nb;
          t += gridDim.x * blockDim.x) {
       const Box2 p = node2_child(nodes[t >> 1], t & 1u);
-      if (!(p.lo[0] <= p.hi[0] && p.lo[1] <= p.hi[1] && p.lo[2] <= p.hi[2])) *irregular = 1u;
+      if (!ordered_box(p.lo, p.hi)) *irregular = 1u;
     }
     return;
   }
@@ -1327,10 +1371,7 @@ __global__ void widen_kernel(const Node2 *__restrict__ nodes,
     for (int k = 0; k < 3; k++)
       ok = ok && p.lo[k] <= q.lo[k] && q.lo[k] <= q.hi[k] && q.hi[k] <= p.hi[k];
     if (!ok) *irregular = 1u;
-    WideRec r;
-    r.a = make_float4(q.lo[0], q.hi[0], q.lo[1], q.hi[1]);
-    r.b = make_float4(q.lo[2], q.hi[2], __uint_as_float(q.ref), __uint_as_float(q.count));
-    wide[t] = r;
+    wide[t] = make_wide(q);
   }
 }
 
@@ -1526,12 +1567,9 @@ srt_status build_kind(srt_accel *a, const float *v, const uint32_t *f,
   } else {
     emit_node2_kernel<KIND><<<gk, kBlock, 0, st>>>(codes, kchild, kflags, krange, flag,
                                                    slot, ibox, a->prims.as<float4>(),
-                                                   scene, kidx, a->nodes.as<Node2>(),
-                                                   ctx->d_err);
+                                                   scene, kidx, kparent, a->nodes.as<Node2>(),
+                                                   a->wide, a->wide_cap, ctx->d_err);
     ctx->launches++;
-    s = build_wide(ctx, a->nodes.as<Node2>(), &scene->nbranches, m, a->wide_cap,
-                   a->wide, &scene->irregular);
-    if (s != SRT_OK) return s;
   }
 #undef ENSURE2
   return cuda_status(cudaGetLastError(), "emit");
