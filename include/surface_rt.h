@@ -154,9 +154,10 @@ typedef struct srt_trace_opts {
  * ties.  Both give identical hits; the default does far less work. */
 #define SRT_TRACE_SINGLE_PASS 1u
 /* Trace the rays in a coherent order (a Morton curve over origin and
- * direction, sorted on the GPU) instead of array order: fewer divergent warps
- * on large ray sets at the cost of the sort.  Hits are identical and are
- * written at each ray's own index. */
+ * direction, sorted on the GPU; from 2^15 rays on, rays that come in rows in
+ * tiles of their rows) instead of array order: fewer divergent warps on large
+ * ray sets at the cost of the order.  Hits are identical and are written at
+ * each ray's own index. */
 #define SRT_TRACE_SORT_RAYS 2u
 /* Launch the first traversal pass as one thread per ray over a grid of all
  * rays instead of the default persistent warps (as many blocks as the GPU
