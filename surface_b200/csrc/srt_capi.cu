@@ -303,6 +303,10 @@ SRT_API srt_status srt_ctx_destroy(srt_ctx *c) {
   if (c->ev_inputs) cudaEventDestroy(c->ev_inputs);
   if (c->ev_free) cudaEventDestroy(c->ev_free);
   if (c->copy_stream) cudaStreamDestroy(c->copy_stream);
+  if (c->nmarks) {  // marches may be under way on their streams
+    cudaDeviceSynchronize();
+    for (int k = 0; k < c->nmarks; k++) cudaFree(c->marks[k].p);
+  }
   // (what a call under way on another stream holds of it goes when that ends)
   if (c->pool) cudaMemPoolDestroy(c->pool);
   if (c->d_err) cudaFree(c->d_err);

@@ -12,6 +12,7 @@
 #include <stdint.h>
 
 #include <atomic>
+#include <mutex>
 #include <string>
 #include <vector>
 
@@ -188,9 +189,19 @@ struct srt_ctx {
       s_stage_in, s_stage_out, s_stage_aux, s_stage_sub, s_stage_scal, s_stage_norm,
       s_defer, s_spawn, s_rkey, s_rorder, s_isect_sub, s_stage_isect, s_keys3, s_vals3,
       s_status, s_lscan, s_rays_in, s_kidx, s_kprefix, s_raster, s_status_lg;
-  // memory of single calls, taken and given back in the order of the call's
-  // stream (vol_brick_kernel's marks); NULL where the device has no such pools
+  // Memory in the order of a stream (vol_brick_kernel's marks); NULL where the
+  // device has no such pools.  The first kMarkStreams streams that march keep a
+  // buffer each, which their calls use one after the other.
+  static constexpr int kMarkStreams = 8;
+  struct MarkBuf {
+    unsigned long long stream = 0;  // its id, which no later stream takes
+    void *p = nullptr;
+    size_t cap = 0;
+  };
   cudaMemPool_t pool = nullptr;
+  std::mutex marks_mu;  // held while a call that uses a buffer is enqueued
+  MarkBuf marks[kMarkStreams];
+  int nmarks = 0;
   uint32_t os_epoch = 0;  // look-back epoch of the last sort pass (srt_sort.cu)
   // recorded after a build's host inputs were copied; the next staged ray
   // array waits for it (inputs_pending)

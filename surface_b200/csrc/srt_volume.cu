@@ -715,6 +715,56 @@ static srt_status vol_view(srt_ctx *ctx, const void *p, size_t bytes, DevBuf &st
   return SRT_OK;
 }
 
+// Memory for a march's brick marks: its stream's buffer (with the lock, so
+// that calls of other threads on that stream come after), or the call's own,
+// to be given back (own), where the stream has none to itself or is captured,
+// so that the graph owns it.  An allocation and its return take 2 us of the
+// stream's time at every call.
+struct Marks {
+  void *p = nullptr;
+  bool own = false;
+  std::unique_lock<std::mutex> lock;
+};
+static Marks take_marks(srt_ctx *ctx, size_t bytes, cudaStream_t st) {
+  Marks m;
+  if (!ctx->pool) return m;
+  cudaStreamCaptureStatus capture = cudaStreamCaptureStatusNone;
+  unsigned long long id = 0;
+  if (cudaStreamIsCapturing(st, &capture) == cudaSuccess &&
+      capture == cudaStreamCaptureStatusNone && cudaStreamGetId(st, &id) == cudaSuccess) {
+    m.lock = std::unique_lock<std::mutex>(ctx->marks_mu);
+    srt_ctx::MarkBuf *b = nullptr;
+    for (int k = 0; k < ctx->nmarks && !b; k++)
+      if (ctx->marks[k].stream == id) b = &ctx->marks[k];
+    if (!b && ctx->nmarks < srt_ctx::kMarkStreams) {
+      b = &ctx->marks[ctx->nmarks++];
+      b->stream = id;
+    }
+    if (b && b->cap < bytes) {
+      size_t cap = (size_t)1 << 16;
+      while (cap < bytes) cap *= 2;
+      void *p = nullptr;
+      if (cudaMallocFromPoolAsync(&p, cap, ctx->pool, st) == cudaSuccess) {
+        if (b->p) cudaFreeAsync(b->p, st);
+        b->p = p;
+        b->cap = cap;
+      }
+    }
+    if (b && b->cap >= bytes) {
+      m.p = b->p;
+      return m;
+    }
+    m.lock.unlock();
+  }
+  cudaGetLastError();
+  m.own = cudaMallocFromPoolAsync(&m.p, bytes, ctx->pool, st) == cudaSuccess;
+  if (!m.own) {
+    cudaGetLastError();
+    m.p = nullptr;  // every sample is marched
+  }
+  return m;
+}
+
 // The texture's sampling state into K; host remap tables are staged in tmp.
 static srt_status apply_sampling(srt_ctx *ctx, const srt_volume_sampling *sm, VolConst &K,
                                  DevBuf (&tmp)[3], cudaStream_t st) {
@@ -811,21 +861,14 @@ SRT_API srt_status srt_volume_march_fwd_ex(srt_ctx *ctx, const srt_volume_params
   // reading of the density and 5 us) and a transparent sample's alpha is 0
   const int3 nb = make_int3((dims[0] - 1) / kBrick + 1, (dims[1] - 1) / kBrick + 1,
                             (dims[2] - 1) / kBrick + 1);
-  uint8_t *occ = nullptr;
+  Marks marks;
   const double samples =
       (double)npix * std::min<double>(params->max_steps, 2.0 / (double)params->step);
   if (samples >= kBrickSamples + 4.0 * (double)nvox * kBrickTexel && params->alpha_max >= 0.0f &&
       std::isfinite(params->sigma_scale) && std::isfinite(params->step) && nb.y < 65536 &&
-      nb.z < 65536 && dims[0] <= (1 << 30) &&  // (texels past a row's end in 32 bits)
-      ctx->pool) {
-    // the call's own marks, in its stream's order: marches may run at the same
-    // time on several streams, and under capture they belong to the graph
-    if (cudaMallocFromPoolAsync(reinterpret_cast<void **>(&occ), (size_t)nb.x * nb.y * nb.z,
-                                ctx->pool, st) != cudaSuccess) {
-      cudaGetLastError();
-      occ = nullptr;  // every sample is marched
-    }
-  }
+      nb.z < 65536 && dims[0] <= (1 << 30))  // (texels past a row's end in 32 bits)
+    marks = take_marks(ctx, (size_t)nb.x * nb.y * nb.z, st);
+  uint8_t *occ = static_cast<uint8_t *>(marks.p);
   if (occ) {
     const auto bricks = K.nremap[0] || K.nremap[1] || K.nremap[2] ? vol_brick_kernel<true>
                                                                   : vol_brick_kernel<false>;
@@ -845,7 +888,8 @@ SRT_API srt_status srt_volume_march_fwd_ex(srt_ctx *ctx, const srt_volume_params
       reinterpret_cast<float4 *>(di), dtr, occ, nb);
   ctx->launches++;
   e = cudaGetLastError();
-  if (occ) cudaFreeAsync(occ, st);
+  if (marks.own) cudaFreeAsync(marks.p, st);
+  if (marks.lock.owns_lock()) marks.lock.unlock();
   if (e != cudaSuccess) return cuda_status(e, "volume fwd");
   if (!img_dev) cudaMemcpyAsync(image, di, npix * 16, cudaMemcpyDeviceToHost, st);
   if (!tr_dev) cudaMemcpyAsync(transmittance, dtr, npix * 4, cudaMemcpyDeviceToHost, st);
